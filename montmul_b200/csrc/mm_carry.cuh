@@ -87,6 +87,36 @@ struct Acc96 {
     __device__ __forceinline__ uint64_t rest() const { return ((uint64_t)a1 << 32) | a0; }  // a2 == 0 here
 };
 
+// A segment's E limbs to or from global memory, 16 bytes at a time when E and the address allow
+// it (the address of every segment is that of segment 0 plus a multiple of 4 E bytes, so the test
+// of one thread's address holds for all). Lanes hold consecutive segments, so single words touch
+// one 32-byte sector per lane per word; as 16-byte words a segment of 16 limbs takes 4 accesses
+// instead of 16.
+template <int E> __device__ __forceinline__ bool seg_aligned(const uint32_t* p) {
+    return E % 4 == 0 && ((uintptr_t)p & 15) == 0;
+}
+template <int E> __device__ __forceinline__ void store_seg(uint32_t* __restrict__ p, const uint32_t (&L)[E]) {
+    if (seg_aligned<E>(p)) {
+#pragma unroll
+        for (int e = 0; e + 3 < E; e += 4) *reinterpret_cast<uint4*>(p + e) = make_uint4(L[e], L[e + 1], L[e + 2], L[e + 3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) p[e] = L[e];
+    }
+}
+template <int E> __device__ __forceinline__ void load_seg(const uint32_t* p, uint32_t (&v)[E]) {
+    if (seg_aligned<E>(p)) {
+#pragma unroll
+        for (int e = 0; e + 3 < E; e += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(p + e);
+            v[e] = q.x; v[e + 1] = q.y; v[e + 2] = q.z; v[e + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = p[e];
+    }
+}
+
 // T = sum C_q 2^(32 q) over the 2n coefficients of a product in natural order (coefficient q < n
 // is re of element q, q >= n is im of element q - n), written to `out` (2n limbs, global).
 // Returns the carry out of the top, which must be 0 for a product that fits.
@@ -116,10 +146,7 @@ __device__ __noinline__ uint64_t carry_product(const F2* s2, const F1* s1, uint3
         for (int e = 0; e < E; ++e) L[e] = 0;
     }
     const uint64_t top = block_resolve<E, TA, NT>(L, c, 0, sc);
-    if (t < TA) {
-#pragma unroll
-        for (int e = 0; e < E; ++e) out[q0 + e] = L[e];
-    }
+    if (t < TA) store_seg<E>(out + q0, L);
     gsync<NT>();
     return top;
 }
@@ -253,10 +280,15 @@ __device__ __noinline__ bool wrap_combine(const F2* s2, const F1* s1, const uint
     constexpr int K = 1 << M, COUNT = K;
     constexpr int E = cmax(2, COUNT / NT), TA = COUNT / E;
     const int t = gtid<NT>();
-    uint32_t L[E];
+    uint32_t L[E], hi32[E];
     uint64_t c = 0;
     const int q0 = t * E;
     if (t < TA) {
+        // T's low half joins the sums here and its high half after the resolution: both loads are
+        // issued together, the second one's latency under the first sum and its barriers.
+        uint32_t lo32[E];
+        load_seg<E>(tl + q0, lo32);
+        load_seg<E>(tl + K + q0, hi32);
         Acc96 acc;
 #pragma unroll
         for (int e = 0; e < E; e += 2) {
@@ -266,12 +298,12 @@ __device__ __noinline__ bool wrap_combine(const F2* s2, const F1* s1, const uint
             const F1 a1 = s1[sj];
             uint32_t w0, w1, w2;
             crt3(a1.re, a2.re, w0, w1, w2);
-            uint64_t lo = (((uint64_t)w1 << 32) | w0) + tl[q0 + e];
-            w2 += lo < (uint64_t)tl[q0 + e];
+            uint64_t lo = (((uint64_t)w1 << 32) | w0) + lo32[e];
+            w2 += lo < (uint64_t)lo32[e];
             L[e] = acc.add_shift((uint32_t)lo, (uint32_t)(lo >> 32), w2);
             crt3(a1.im, a2.im, w0, w1, w2);
-            lo = (((uint64_t)w1 << 32) | w0) + tl[q0 + e + 1];
-            w2 += lo < (uint64_t)tl[q0 + e + 1];
+            lo = (((uint64_t)w1 << 32) | w0) + lo32[e + 1];
+            w2 += lo < (uint64_t)lo32[e + 1];
             L[e + 1] = acc.add_shift((uint32_t)lo, (uint32_t)(lo >> 32), w2);
         }
         c = acc.rest();
@@ -287,17 +319,14 @@ __device__ __noinline__ bool wrap_combine(const F2* s2, const F1* s1, const uint
         uint64_t acc = 0;
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            acc += (uint64_t)L[e] + tl[K + q0 + e];
+            acc += (uint64_t)L[e] + hi32[e];
             L[e] = (uint32_t)acc;
             acc >>= 32;
         }
         c = acc;
     }
     top = block_resolve<E, TA, NT>(L, c, 0, sc);
-    if (t < TA) {
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[q0 + e] = L[e];
-    }
+    if (t < TA) store_seg<E>(x + q0, L);
     gsync<NT>();
     return top == 0;
 }
