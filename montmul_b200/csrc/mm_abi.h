@@ -52,7 +52,7 @@ struct GArgs {
     F1* w1;
     int m;    // log2 n
 };
-typedef void (*GStepFn)(GArgs, uint32_t, uint32_t);
+typedef void (*GStepFn)(GArgs, uint32_t, uint32_t, const uint2*);
 typedef void (*GMulFn)(GArgs, uint32_t, uint32_t, uint32_t, F2*, F1*);
 typedef void (*GSetupFn)(GArgs, const uint32_t*, const uint32_t*, F2*, F1*, F2, F1, uint32_t, const uint32_t*);   // k, plain in g.a
 struct GlobalKernels {
@@ -72,8 +72,13 @@ constexpr int kMinClusterLogN = 14;
 constexpr int kMaxClusterLogN = 15;
 constexpr int kClusterChunkLog = 13;        // the default chunk
 constexpr int kClusterPairChunkLog = 12;    // the two-blocks-per-SM chunk, at L = 32768
+// kClusterWideLogN (L = 131072, eight blocks): not a mode a schedule names; run takes it for
+// wraparound batches in global mode (mm_backend.cu).
+constexpr int kClusterWideLogN = 16;
 int cluster_configure();
-int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t slots, uint32_t bits, void* stream);
+// One cluster per slot, `bits` steps each; with items, one per item (slot, steps).
+int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, void* stream);
+int cluster_capacity(int m, int chunk_log, int* clusters);   // clusters resident at once
 // Enqueues wait_check_kernel (mm_global.cuh) on a stream; non-zero if the launch failed.
 int launch_wait_check(uint32_t* err, uint64_t limit_ns, void* stream);   // mm_global.cu
 

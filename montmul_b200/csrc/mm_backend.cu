@@ -279,6 +279,32 @@ int check_err(mm_b200_batch* b, const char* what) {
     return MM_OK;
 }
 
+// Cluster mode of a global batch: the shared-layout tables of its length and the kernels' shared
+// memory opt-in (once per device).
+int ensure_cluster(mm_b200_batch* b) {
+    if (!b->ctab) {
+        const DevTables* t = nullptr;
+        int rc = ensure_tables(b->dev, b->m, false, &t);
+        if (rc) return rc;
+        b->ctab = t;
+    }
+    std::lock_guard<std::mutex> lock(b->dev->mu);
+    if (!b->dev->cluster_configured) {
+        const int e = cluster_configure();
+        if (e) return fail(MM_ERR_CUDA, std::string("cluster mode: ") + cudaGetErrorString((cudaError_t)e));
+        b->dev->cluster_configured = true;
+    }
+    return MM_OK;
+}
+
+// L = 131072 in global mode can also step in clusters of eight blocks (mm_cluster.cuh), the vector in
+// their shared memory, where global mode takes one block per slot and streams it through HBM. A
+// device holds 18 such clusters, 432 us a step, so 24 us per slot-step at any number of slots;
+// global mode takes 4.1 ms a step for up to one slot per SM and 22 us per slot-step from two per
+// SM on. The clusters are faster up to one slot per SM (24 slots x 8 steps: 35.2 -> 6.9 ms) and
+// slower beyond. The plain REDC path has no cluster form; the mixed launch's items stay in global mode.
+bool cluster_capable(const mm_b200_batch* b) { return b->global && !b->cluster && b->m == kClusterWideLogN && !b->plain; }
+
 int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     size_t most = 0;
     for (size_t i = 0; i < b->slots; ++i) most = std::max(most, (size_t)(b->nbits[i] - b->pos[i]));
@@ -293,17 +319,24 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         g = global_args(b);
         g.a.bare = a.bare;
     }
+    size_t active = 0;
+    for (size_t i = 0; i < b->slots; ++i) active += b->pos[i] < b->nbits[i];
+    const bool clustered = b->cluster || (cluster_capable(b) && active <= (size_t)b->dev->sms);
+    if (clustered) {
+        rc = ensure_cluster(b);
+        if (rc) return rc;
+    }
     const size_t chunk = (size_t)std::max(1, b->sched.launch_steps > 0 ? b->sched.launch_steps : b->dev->max_launch_steps);
     while (left > 0) {
         const uint32_t s = (uint32_t)std::min(left, chunk);
-        if (b->cluster) {
+        if (clustered) {
             SlotArgs c = a;
             c.tab2 = b->ctab->t2;
             c.tab1 = b->ctab->t1;
-            const int e = cluster_launch(b->m, b->cluster_chunk_log, c, (uint32_t)b->slots, s, b->stream);
+            const int e = cluster_launch(b->m, b->cluster_chunk_log, c, (uint32_t)b->slots, s, nullptr, b->stream);
             if (e) return fail(MM_ERR_CUDA, std::string("cluster launch: ") + cudaGetErrorString((cudaError_t)e));
         } else if (b->global) {
-            b->gk.step<<<(unsigned)b->slots, b->gk.threads, b->gk.smem, b->stream>>>(g, 0, s);
+            b->gk.step<<<(unsigned)b->slots, b->gk.threads, b->gk.smem, b->stream>>>(g, 0, s, nullptr);
         } else {
             b->step_fn<<<(unsigned)b->slots, b->step_threads, b->ks.smem, b->stream>>>(a, 0, s, nullptr);
         }
@@ -328,24 +361,6 @@ int ensure_global_buffers(mm_b200_batch* b) {
     if (!b->d_w2) {
         MM_CK(cudaMalloc(&b->d_w2, b->slots * b->n * sizeof(F2)));
         MM_CK(cudaMalloc(&b->d_w1, b->slots * b->n * sizeof(F1)));
-    }
-    return MM_OK;
-}
-
-// Cluster mode of a global batch: the shared-layout tables of its length and the kernels' shared
-// memory opt-in (once per device).
-int ensure_cluster(mm_b200_batch* b) {
-    if (!b->ctab) {
-        const DevTables* t = nullptr;
-        int rc = ensure_tables(b->dev, b->m, false, &t);
-        if (rc) return rc;
-        b->ctab = t;
-    }
-    std::lock_guard<std::mutex> lock(b->dev->mu);
-    if (!b->dev->cluster_configured) {
-        const int e = cluster_configure();
-        if (e) return fail(MM_ERR_CUDA, std::string("cluster mode: ") + cudaGetErrorString((cudaError_t)e));
-        b->dev->cluster_configured = true;
     }
     return MM_OK;
 }
@@ -582,6 +597,10 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     b->gk = global_kernels();
     b->sched.threads = global ? b->gk.threads : (m <= kMaxSharedLogN ? threads_for(m) : 0);
     b->gtab = gtab;
+    if (cluster_capable(b.get())) {
+        rc = ensure_cluster(b.get());
+        if (rc) return rc;
+    }
     if (m <= kMaxSharedLogN) {
         kernel_set(m, b->ks);
         b->step_fn = b->ks.step;

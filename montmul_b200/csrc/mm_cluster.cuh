@@ -1,5 +1,5 @@
 // Cluster mode: lengths whose vector exceeds one SM's shared memory but fits a thread-block
-// cluster's. n = 2^M elements (M = 14, 15: L = 32768, 65536) are spread over C = n / 8192 CTAs
+// cluster's. n = 2^M elements (M = 14, 15, 16: L = 32768 to 131072) are spread over C = n / 8192 CTAs
 // of one cluster, 8,192 elements (192 KiB, the F2 then F1 arrays at swz positions) in each CTA's
 // shared memory; the CTAs reach each other's chunks through distributed shared memory. The
 // reference runs these lengths in global memory (kernels/src/lib.rs:455-511); here nothing of
@@ -391,8 +391,7 @@ __device__ __noinline__ uint64_t cl_carry_product(const Chunks<C>& ch, uint32_t*
         L[e] = acc.add_shift(w0, w1, w2);
     }
     const uint64_t top = cluster_resolve<E, NT, C>(L, acc.rest(), 0, sc, cc, cl);
-#pragma unroll
-    for (int e = 0; e < E; ++e) out[q0 + e] = L[e];
+    store_seg<E>(out + q0, L);
     return top;
 }
 
@@ -434,7 +433,9 @@ __device__ __noinline__ bool cl_wrap_combine(const F2* s2, const F1* s1, const u
     constexpr int K = 1 << M, CL = M - ilog2c(C), E = (1 << CL) / NT;
     const int l0 = (int)threadIdx.x * E;
     const int q0 = (int)cl.block_rank() * (1 << CL) + l0;
-    uint32_t L[E];
+    uint32_t L[E], lo32[E], hi32[E];
+    load_seg<E>(tl + q0, lo32);
+    load_seg<E>(tl + K + q0, hi32);
     Acc96 acc;
 #pragma unroll
     for (int e = 0; e < E; e += 2) {
@@ -443,12 +444,12 @@ __device__ __noinline__ bool cl_wrap_combine(const F2* s2, const F1* s1, const u
         const F1 a1 = s1[sj];
         uint32_t w0, w1, w2;
         crt3(a1.re, a2.re, w0, w1, w2);
-        uint64_t lo = (((uint64_t)w1 << 32) | w0) + tl[q0 + e];
-        w2 += lo < (uint64_t)tl[q0 + e];
+        uint64_t lo = (((uint64_t)w1 << 32) | w0) + lo32[e];
+        w2 += lo < (uint64_t)lo32[e];
         L[e] = acc.add_shift((uint32_t)lo, (uint32_t)(lo >> 32), w2);
         crt3(a1.im, a2.im, w0, w1, w2);
-        lo = (((uint64_t)w1 << 32) | w0) + tl[q0 + e + 1];
-        w2 += lo < (uint64_t)tl[q0 + e + 1];
+        lo = (((uint64_t)w1 << 32) | w0) + lo32[e + 1];
+        w2 += lo < (uint64_t)lo32[e + 1];
         L[e + 1] = acc.add_shift((uint32_t)lo, (uint32_t)(lo >> 32), w2);
     }
     uint64_t top = cluster_resolve<E, NT, C>(L, acc.rest(), 0, sc, cc, cl);
@@ -457,13 +458,12 @@ __device__ __noinline__ bool cl_wrap_combine(const F2* s2, const F1* s1, const u
     uint64_t a2 = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        a2 += (uint64_t)L[e] + tl[K + q0 + e];
+        a2 += (uint64_t)L[e] + hi32[e];
         L[e] = (uint32_t)a2;
         a2 >>= 32;
     }
     top = cluster_resolve<E, NT, C>(L, a2, 0, sc, cc, cl);
-#pragma unroll
-    for (int e = 0; e < E; ++e) x[q0 + e] = L[e];
+    store_seg<E>(x + q0, L);
     return top == 0;
 }
 
@@ -531,36 +531,54 @@ __device__ __forceinline__ void cl_step_slot(const SlotArgs& a, uint32_t slot, u
 }
 
 // The uniform cluster launch: cluster i (C = 2^(M - CL) consecutive blocks of 2^CL elements)
-// steps slot first + i. CL = 13: one block of 192 KiB per SM; CL = 12 (L = 32768 only): two
+// steps slot first + i, or with an item list item i's (slot, steps). CL = 13: one block of 192 KiB per SM; CL = 12 (L = 32768 only): two
 // blocks of 96 KiB per SM, so twice the warps hide the latency of the cross-block accesses, at
 // 64 registers per thread and with more of each cross-block pass remote.
 template <int M, int CL>
 __global__ void __launch_bounds__(kClusterThreads, kChunkLog - CL + 1)
-    cluster_step_kernel(SlotArgs a, uint32_t first, uint32_t bits) {
+    cluster_step_kernel(SlotArgs a, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
     constexpr int C = 1 << (M - CL);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<kClusterThreads>::words];
     __shared__ ClusterCarry cc;
-    cl_step_slot<M, kClusterThreads, C>(a, first + blockIdx.x / C, bits, smem_raw, sc, &cc);
+    uint32_t slot = first + blockIdx.x / C;
+    if (items) {
+        const uint2 it = items[blockIdx.x / C];
+        slot = it.x;
+        bits = it.y;
+    }
+    cl_step_slot<M, kClusterThreads, C>(a, slot, bits, smem_raw, sc, &cc);
 }
 
 // ---- host side: launch and shared-memory opt-in of one instantiation ----
-template <int M, int CL>
-cudaError_t launch_cluster_m(const SlotArgs& a, uint32_t slots, uint32_t bits, cudaStream_t s) {
-    constexpr int C = 1 << (M - CL);
+struct ClusterLaunch {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C * slots, 1, 1);
-    cfg.blockDim = dim3(kClusterThreads, 1, 1);
-    cfg.dynamicSmemBytes = 24 << CL;
-    cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cluster_step_kernel<M, CL>, a, 0u, bits);
+    ClusterLaunch(int c, uint32_t slots, int smem, cudaStream_t s) {
+        cfg.gridDim = dim3(c * slots, 1, 1);
+        cfg.blockDim = dim3(kClusterThreads, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+template <int M, int CL>
+cudaError_t launch_cluster_m(const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, cudaStream_t s) {
+    const ClusterLaunch l(1 << (M - CL), slots, 24 << CL, s);
+    return cudaLaunchKernelEx(&l.cfg, cluster_step_kernel<M, CL>, a, 0u, bits, items);
+}
+
+// Clusters the current device holds at once.
+template <int M, int CL>
+cudaError_t capacity_cluster_m(int* clusters) {
+    const ClusterLaunch l(1 << (M - CL), 1, 24 << CL, nullptr);
+    return cudaOccupancyMaxActiveClusters(clusters, cluster_step_kernel<M, CL>, &l.cfg);
 }
 
 template <int M, int CL>
@@ -571,6 +589,7 @@ cudaError_t configure_cluster_m() {
 
 // The 4,096-element-chunk instantiation at L = 32768 (mm_cluster_half.cu).
 cudaError_t cluster_half_chunk_configure();
-cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t slots, uint32_t bits, cudaStream_t s);
+cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, cudaStream_t s);
+cudaError_t cluster_half_chunk_capacity(int* clusters);
 
 }  // namespace mm

@@ -56,12 +56,15 @@ MM_HD constexpr int swz_c(int e) {
 // ---- pass schedule: radices, DIF order ----
 // m = log2 n. m = 3a -> [8]*a; m = 3a + 1 -> [4, 4, 8*(a-1)]; m = 3a + 2 -> [4, 8*a];
 // m = 1 -> [2], m = 2 -> [4]. Radix-8 passes dominate; the last DIF pass (span 1) carries no
-// twiddles, so it is kept at radix 8 whenever m >= 3.
+// twiddles, so it is kept at radix 8 whenever m >= 3. m = 16, which only a cluster of eight blocks
+// runs (mm_cluster.cuh), is [8, 4, 4, 8, 8, 8]: after a radix-8 first pass every group lies inside
+// one block's 8,192 elements, after a radix-4 one it would not.
 MM_HD constexpr int sched_passes(int m) {
     return m <= 3 ? 1 : (m % 3 == 0 ? m / 3 : (m % 3 == 1 ? m / 3 + 1 : m / 3 + 1));
 }
 MM_HD constexpr int sched_radix(int m, int i) {
     return m == 1 ? 2 : m == 2 ? 4 : m == 3 ? 8
+         : m == 16 ? (i == 1 || i == 2 ? 4 : 8)
          : (m % 3 == 0 ? 8 : (m % 3 == 1 ? (i < 2 ? 4 : 8) : (i < 1 ? 4 : 8)));
 }
 MM_HD constexpr int ilog2c(int v) { return v <= 1 ? 0 : 1 + ilog2c(v / 2); }

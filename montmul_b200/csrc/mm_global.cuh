@@ -384,8 +384,7 @@ __device__ __forceinline__ uint64_t chunked_sum(const COEF& coef, int count, uin
             L[e] = acc.add_shift(w0, w1, w2);
         }
         cin = block_resolve<kChunkE, NT, NT>(L, acc.rest(), cin, sc);
-#pragma unroll
-        for (int e = 0; e < kChunkE; ++e) out[q0 + e] = L[e];
+        store_seg<kChunkE>(out + q0, L);
     }
     gsync<NT>();
     return cin;
@@ -620,16 +619,22 @@ __device__ __forceinline__ bool gstep_slot(const GArgs& g, uint32_t slot, uint32
     return st != kStepTimeout;
 }
 
-// The uniform launch, global mode: one block per slot first + blockIdx.x.
+// The uniform launch, global mode: one block per slot first + blockIdx.x, or per item (slot, steps).
 template <int NT>
-__global__ void __launch_bounds__(NT, 2) gstep_kernel(GArgs g, uint32_t first, uint32_t bits) {
+__global__ void __launch_bounds__(NT, 2) gstep_kernel(GArgs g, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<NT>::words];
     __shared__ uint64_t bars[2];
     const TileSmem sm{smem_raw, bars};
     tile_init<NT>(sm);
     uint32_t par = 0;
-    gstep_slot<NT>(g, first + blockIdx.x, bits, sm, sc, par);
+    uint32_t slot = first + blockIdx.x;
+    if (items) {
+        const uint2 it = items[blockIdx.x];
+        slot = it.x;
+        bits = it.y;
+    }
+    gstep_slot<NT>(g, slot, bits, sm, sc, par);
 }
 
 // x[out] <- x[ia] x[ib] R^-1, global mode; spec: n-element scratch for F(x[ib]).

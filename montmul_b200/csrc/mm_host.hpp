@@ -114,11 +114,14 @@ template <class E> inline void gen_transform(int m, bool weighted, E* t) {
         for (int k = w0 ? 0 : 1; k < R; ++k) {
             const int row = w0 ? k : k - 1;
             const uint64_t rk = (uint64_t)rev_bits(k, lr);
+            E fs = gpow(W, rk), bs = gpow(V, rk);
+            if (w0) { fs = Gf<E>::mul(fs, zeta); bs = Gf<E>::mul(bs, zi); }
+            E fw = one<E>(), bw = one<E>();   // (W^rk zeta)^j and (V^rk / zeta)^j
             for (int j = 0; j < q; ++j) {
-                E fw = gpow(W, rk * j), bw = gpow(V, rk * j);
-                if (w0) { fw = Gf<E>::mul(fw, gpow(zeta, j)); bw = Gf<E>::mul(bw, gpow(zi, j)); }
                 f[row * q + j] = fw;
                 b[row * q + j] = bw;
+                fw = Gf<E>::mul(fw, fs);
+                bw = Gf<E>::mul(bw, bs);
             }
         }
     }
@@ -142,10 +145,13 @@ template <class E> inline std::vector<E> gen_length_tables(int m) {
     roots<E>(m, omega, zeta);
     const E wi = Gf<E>::inv(omega);
     const int h = 1 << (m - 1);
-    for (int p = 0; p < h; ++p) {
-        const int r = rev_bits(p, m - 1);
-        t[lt_unpack_off(m) + p] = gpow(omega, (uint64_t)r);
-        t[lt_unpack_off(m) + h + p] = gpow(wi, (uint64_t)r);
+    E a = one<E>(), b = one<E>();   // omega^r and omega^-r
+    for (int r = 0; r < h; ++r) {
+        const int p = rev_bits(r, m - 1);
+        t[lt_unpack_off(m) + p] = a;
+        t[lt_unpack_off(m) + h + p] = b;
+        a = Gf<E>::mul(a, omega);
+        b = Gf<E>::mul(b, wi);
     }
     return t;
 }

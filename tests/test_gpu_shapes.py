@@ -1,0 +1,44 @@
+"""The shapes run chooses by itself (no counterpart in the reference): clusters of eight blocks at
+L = 131072. Raw limbs equal those of the same batch stepped another way."""
+import random
+
+import numpy as np
+import pytest
+
+from montmul_b200 import ModBatch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    from montmul_b200 import B200
+    return B200()
+
+
+def batch(gpu, bits, slots, nbits, base=3, seed=1):
+    """Odd moduli of `bits` bits (the last one 2^bits - 1), random values, exponents of nbits[i] bits."""
+    rng = random.Random(f"{bits} {slots} {seed}")
+    mods = [rng.getrandbits(bits) | (1 << (bits - 1)) | 1 for _ in range(slots - 1)] + [(1 << bits) - 1]
+    b = ModBatch(gpu, mods, base)
+    for i, n in enumerate(mods):
+        b.load_raw(i, 2 * n - 1 if i == slots - 1 else rng.randrange(2 * n))
+        b.set_exponent(i, rng.getrandbits(nbits[i]) | (1 << (nbits[i] - 1)) if nbits[i] else 0)
+    return b
+
+
+def raw(b):
+    be, st = b.backend_and_state()
+    return np.array(be.read_all(st))
+
+
+def test_clusters_of_eight_same_raw_as_global_mode(gpu):
+    """L = 131072: run takes clusters of eight blocks, a plan's items run in global mode."""
+    from montmul_b200.backend import Plan
+    for bits in (1_048_574, 2_097_148):
+        a, b = batch(gpu, bits, 2, [6, 4]), batch(gpu, bits, 2, [6, 4])
+        a.run(6)
+        plan = Plan([b], 6)
+        plan.run(6)
+        plan.close()
+        assert a.params.len == 131072 and np.array_equal(raw(a), raw(b))
