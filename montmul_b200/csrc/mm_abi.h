@@ -33,10 +33,18 @@ typedef void (*SetupFn)(const uint32_t*, const uint32_t*, F2*, F1*, const F2K*, 
                         const uint32_t*, uint32_t, int);
 typedef void (*TransformFn)(F2*, F1*, const F2K*, const F1*, uint32_t, int);
 
+// A step kernel with more threads per slot, for batches that leave SMs idle (nullptr: none).
+struct WideShape {
+    StepFn step;
+    int threads;
+};
+constexpr int kWideShapes = 2;   // widest first
+
 struct KernelSet {
     StepFn step;
     StepFn step_alt;         // the alternative block shape of this length's step (nullptr: none)
     int threads_alt;
+    WideShape wide[kWideShapes];
     MulFn mul;
     SetupFn setup;
     TransformFn transform;   // the Transform trait's forward / inverse (shared memory)
@@ -140,6 +148,13 @@ constexpr int threads_for(int m) {
 // SM; 0 threads: none): the runner-up of the shapes measured at full occupancy, 4,096 <= L <= 16,384.
 constexpr int alt_threads_for(int m) { return m == 11 ? 256 : (m == 12 ? 256 : (m == 13 ? 1024 : 0)); }
 constexpr int alt_min_blocks_for(int m) { return m == 11 ? 4 : (m == 12 ? 2 : 1); }
+
+// The wide shapes of a length, widest first: 4 and 2 times threads_for's threads up to 512 (0: none),
+// at 128 registers a thread. Below 64 elements there is nothing to spread; from L = 8,192 on one
+// block already has 512 threads.
+constexpr int wide_threads_for(int m, int i) {
+    return m < 6 || m > 11 ? 0 : (4 >> i) * threads_for(m) <= 512 ? (4 >> i) * threads_for(m) : 0;
+}
 
 // Defined in mm_inst.cu for each m in [kMinLogN, kMaxSharedLogN].
 #define MM_DECLARE_KERNELS(M) KernelSet kernels_m##M();

@@ -80,6 +80,7 @@ struct mm_b200_device {
     std::mutex mu;
     std::map<int, DevTables> tables;
     std::map<int, bool> configured;
+    std::map<const void*, int> resident;   // blocks of a step kernel that the device holds at once
 };
 
 struct mm_b200_batch {
@@ -90,6 +91,7 @@ struct mm_b200_batch {
     KernelSet ks{};
     StepFn step_fn = nullptr;  // the step kernel of the schedule's block shape (ks.step or ks.step_alt)
     int step_threads = 0;
+    bool step_fixed = false;   // the schedule names the block shape: no wide shape in its place
     bool global = false;       // vector in HBM, tiles through shared memory (mm_global.cuh)
     bool cluster = false;      // global batch stepped in cluster mode (mm_cluster.cuh)
     int cluster_chunk_log = kClusterChunkLog;   // elements per block of the cluster: 2^13 or 2^12
@@ -170,9 +172,10 @@ int ensure_tables(mm_b200_device* dev, int m, bool global, const DevTables** out
         MM_CK(cudaFuncSetAttribute((const void*)ks.transform, cudaFuncAttributeMaxDynamicSharedMemorySize, ks.smem));
         MM_CK(cudaFuncSetAttribute((const void*)ks.step, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
-        if (ks.step_alt) {
-            MM_CK(cudaFuncSetAttribute((const void*)ks.step_alt, cudaFuncAttributeMaxDynamicSharedMemorySize, ks.smem));
-            MM_CK(cudaFuncSetAttribute((const void*)ks.step_alt, cudaFuncAttributePreferredSharedMemoryCarveout,
+        for (StepFn f : {ks.step_alt, ks.wide[0].step, ks.wide[1].step}) {
+            if (!f) continue;
+            MM_CK(cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, ks.smem));
+            MM_CK(cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        cudaSharedmemCarveoutMaxShared));
         }
         dev->configured[m] = true;
@@ -305,6 +308,45 @@ int ensure_cluster(mm_b200_batch* b) {
 // slower beyond. The plain REDC path has no cluster form; the mixed launch's items stay in global mode.
 bool cluster_capable(const mm_b200_batch* b) { return b->global && !b->cluster && b->m == kClusterWideLogN && !b->plain; }
 
+// Blocks of a shared-memory step kernel that the batch's device holds at once.
+int resident_blocks(mm_b200_batch* b, StepFn fn, int threads, int* out) {
+    std::lock_guard<std::mutex> lock(b->dev->mu);
+    auto it = b->dev->resident.find((const void*)fn);
+    if (it == b->dev->resident.end()) {
+        int per = 0;
+        MM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, b->ks.smem));
+        it = b->dev->resident.emplace((const void*)fn, per * b->dev->sms).first;
+    }
+    *out = it->second;
+    return MM_OK;
+}
+
+// The block shape of run's launches over `active` slots in shared memory: the widest one whose
+// blocks are all resident at once, at most five per SM, unless the schedule fixes the shape. With
+// every slot resident the time of a run is one slot's, which more threads shorten (ms for 500 steps
+// at L = 512, default 32 threads -> wide: 64 slots 22.5 -> 14.5, 592 slots 23.4 -> 16.8; 300 steps at L = 1024,
+// 592 slots: 18.2 -> 13.7; 200 steps at L = 4096, 148 slots: 13.8 -> 10.7). With more slots the default
+// shape's rate per SM is higher (L = 512, 64 threads: 700 slots 24 -> 18.1, 1,000 slots 24.2 -> 26.8).
+// Item lists (run_items) keep the default shape: a serving loop runs several of them at the same
+// time, which fill the SMs together.
+int step_shape(mm_b200_batch* b, size_t active, StepFn* fn, int* threads) {
+    *fn = b->step_fn;
+    *threads = b->step_threads;
+    if (b->step_fixed) return MM_OK;
+    for (const WideShape& w : b->ks.wide) {
+        if (!w.step) continue;
+        int res = 0;
+        const int rc = resident_blocks(b, w.step, w.threads, &res);
+        if (rc) return rc;
+        if (active <= (size_t)std::min(res, 5 * b->dev->sms)) {
+            *fn = w.step;
+            *threads = w.threads;
+            return MM_OK;
+        }
+    }
+    return MM_OK;
+}
+
 int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     size_t most = 0;
     for (size_t i = 0; i < b->slots; ++i) most = std::max(most, (size_t)(b->nbits[i] - b->pos[i]));
@@ -326,6 +368,12 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         rc = ensure_cluster(b);
         if (rc) return rc;
     }
+    StepFn step_fn = nullptr;
+    int step_threads = 0;
+    if (!b->global) {
+        rc = step_shape(b, active, &step_fn, &step_threads);
+        if (rc) return rc;
+    }
     const size_t chunk = (size_t)std::max(1, b->sched.launch_steps > 0 ? b->sched.launch_steps : b->dev->max_launch_steps);
     while (left > 0) {
         const uint32_t s = (uint32_t)std::min(left, chunk);
@@ -338,7 +386,7 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         } else if (b->global) {
             b->gk.step<<<(unsigned)b->slots, b->gk.threads, b->gk.smem, b->stream>>>(g, 0, s, nullptr);
         } else {
-            b->step_fn<<<(unsigned)b->slots, b->step_threads, b->ks.smem, b->stream>>>(a, 0, s, nullptr);
+            step_fn<<<(unsigned)b->slots, step_threads, b->ks.smem, b->stream>>>(a, 0, s, nullptr);
         }
         MM_CK(cudaGetLastError());
         ++b->launches;
@@ -919,6 +967,7 @@ int mm_b200_set_schedule(mm_b200_batch* b, const mm_b200_schedule* sc) {
     if (!global) {
         b->step_fn = fn;
         b->step_threads = threads;
+        b->step_fixed = sc->threads != 0;
     }
     b->sched = *sc;
     b->sched.global = cluster ? 2 : (global ? 1 : 0);

@@ -455,9 +455,7 @@ __device__ __noinline__ bool g_wrap_combine(const F2* v2, const F1* v1, int n, c
 // The half-pointwise step over the h-element vector in global memory (pairs cross tiles).
 template <int NT>
 __device__ __noinline__ void half_pointwise_rt(F2* v2, F1* v1, int H, const F2* __restrict__ ab2, const F1* __restrict__ ab1) {
-#pragma unroll 1
-    for (int tau = gtid<NT>(); tau < H / 2 + 1; tau += NT) half_pointwise_pair(v2, v1, H, ab2, ab1, tau);
-    gsync<NT>();
+    half_pointwise_all<NT, false>(v2, v1, H, ab2, ab1);
 }
 
 // ---- the REDC without the wraparound path on global vectors ----

@@ -20,9 +20,20 @@ struct AltStep<M, 0> {
     static StepFn fn() { return nullptr; }
 };
 
+template <int M, int NTW>
+struct WideStep {
+    static StepFn fn() { return step_kernel<M, NTW, 512 / NTW, true>; }   // 128 registers a thread
+};
+template <int M>
+struct WideStep<M, 0> {
+    static StepFn fn() { return nullptr; }
+};
+
 KernelSet MM_CAT(kernels_m, MM_M)() {
     constexpr int NT = threads_for(MM_M), NTA = alt_threads_for(MM_M);
-    return KernelSet{step_kernel<MM_M, NT>, AltStep<MM_M, NTA>::fn(), NTA, mul_kernel<MM_M, NT>, setup_kernel<MM_M, NT>,
+    constexpr int W0 = wide_threads_for(MM_M, 0), W1 = wide_threads_for(MM_M, 1);
+    return KernelSet{step_kernel<MM_M, NT>, AltStep<MM_M, NTA>::fn(), NTA,
+                     {{WideStep<MM_M, W0>::fn(), W0}, {WideStep<MM_M, W1>::fn(), W1}}, mul_kernel<MM_M, NT>, setup_kernel<MM_M, NT>,
                      transform_kernel<MM_M, NT>, NT,
                      smem_bytes<MM_M>()};
 }

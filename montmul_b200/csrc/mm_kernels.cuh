@@ -66,41 +66,58 @@ template <int M> struct SpecStoreOp {
 // index (h - rev(p)) mod h; in place, one thread per pair {p, q} (q = 3 * 2^a - 1 - p for p in
 // octave [2^a, 2^(a+1)), q = p for p < 2). The vector (h elements at swz(p)) may be in shared
 // or global memory.
-__device__ __forceinline__ void half_pointwise_pair(F2* s2, F1* s1, int H, const F2* __restrict__ ab2,
-                                                    const F1* __restrict__ ab1, int tau) {
-    const int p = tau < 2 ? tau : tau - 1 + (1 << (31 - __clz(tau - 1)));
-    const int q = p == 0 ? 0 : (3 << (31 - __clz(p))) - 1 - p;
-    {
-        // e = z_p + conj z_q, d = z_p - conj z_q on reduced values, then e A + d B.
-        const F2 zp = s2[swz(p)], zq = s2[swz(q)];
-        const F2 e = lcfold(f2(zp.re + zq.re, zp.im + lsub<2>(0, zq.im)));
-        const F2 d = lcfold(f2(lsub<2>(zp.re, zq.re), zp.im + zq.im));
-        const F2 op = lcfold(lcadd(lkmulc(e, ab2[p]), lkmulc(d, ab2[H + p])));
-        if (q != p) {
-            const F2 e2 = lcfold(f2(zq.re + zp.re, zq.im + lsub<2>(0, zp.im)));
-            const F2 d2 = lcfold(f2(lsub<2>(zq.re, zp.re), zq.im + zp.im));
-            s2[swz(q)] = lcfold(lcadd(lkmulc(e2, ab2[q]), lkmulc(d2, ab2[H + q])));
-        }
-        s2[swz(p)] = op;
+__device__ __forceinline__ void half_pair(int tau, int& p, int& q) {
+    p = tau < 2 ? tau : tau - 1 + (1 << (31 - __clz(tau - 1)));
+    q = p == 0 ? 0 : (3 << (31 - __clz(p))) - 1 - p;
+}
+__device__ __forceinline__ void half_pointwise_pair(F2* s2, int H, const F2* __restrict__ ab2, int tau) {
+    int p, q;
+    half_pair(tau, p, q);
+    // e = z_p + conj z_q, d = z_p - conj z_q on reduced values, then e A + d B.
+    const F2 zp = s2[swz(p)], zq = s2[swz(q)];
+    const F2 e = lcfold(f2(zp.re + zq.re, zp.im + lsub<2>(0, zq.im)));
+    const F2 d = lcfold(f2(lsub<2>(zp.re, zq.re), zp.im + zq.im));
+    const F2 op = lcfold(lcadd(lkmulc(e, ab2[p]), lkmulc(d, ab2[H + p])));
+    if (q != p) {
+        const F2 e2 = lcfold(f2(zq.re + zp.re, zq.im + lsub<2>(0, zp.im)));
+        const F2 d2 = lcfold(f2(lsub<2>(zq.re, zp.re), zq.im + zp.im));
+        s2[swz(q)] = lcfold(lcadd(lkmulc(e2, ab2[q]), lkmulc(d2, ab2[H + q])));
     }
-    {
-        const F1 zp = s1[swz(p)], zq = s1[swz(q)];
-        const F1 e = cadd(zp, cconj(zq)), d = csub(zp, cconj(zq));
-        const F1 op = cadd(cmul(e, ab1[p]), cmul(d, ab1[H + p]));
-        if (q != p) {
-            const F1 e2 = cadd(zq, cconj(zp)), d2 = csub(zq, cconj(zp));
-            s1[swz(q)] = cadd(cmul(e2, ab1[q]), cmul(d2, ab1[H + q]));
-        }
-        s1[swz(p)] = op;
+    s2[swz(p)] = op;
+}
+__device__ __forceinline__ void half_pointwise_pair(F1* s1, int H, const F1* __restrict__ ab1, int tau) {
+    int p, q;
+    half_pair(tau, p, q);
+    const F1 zp = s1[swz(p)], zq = s1[swz(q)];
+    const F1 e = cadd(zp, cconj(zq)), d = csub(zp, cconj(zq));
+    const F1 op = cadd(cmul(e, ab1[p]), cmul(d, ab1[H + p]));
+    if (q != p) {
+        const F1 e2 = cadd(zq, cconj(zp)), d2 = csub(zq, cconj(zp));
+        s1[swz(q)] = cadd(cmul(e2, ab1[q]), cmul(d2, ab1[H + q]));
     }
+    s1[swz(p)] = op;
 }
 
-template <int MH, int NT>
+// Pairs 0 and 1 (p = q: half a pair's work each) go to the same thread, so H/2 items cover all.
+template <int NT, bool SPLIT>
+__device__ __forceinline__ void half_pointwise_all(F2* s2, F1* s1, int H, const F2* __restrict__ ab2, const F1* __restrict__ ab1) {
+    for_groups<NT, SPLIT>(
+        H / 2,
+        [&](int i) {
+            if (i == 0) half_pointwise_pair(s2, H, ab2, 0);
+            half_pointwise_pair(s2, H, ab2, i + 1);
+        },
+        [&](int i) {
+            if (i == 0) half_pointwise_pair(s1, H, ab1, 0);
+            half_pointwise_pair(s1, H, ab1, i + 1);
+        });
+    gsync<NT>();
+}
+
+template <int MH, int NT, bool SP = false>
 __device__ __noinline__ void half_pointwise(F2* s2, F1* s1, const F2* __restrict__ ab2, const F1* __restrict__ ab1) {
     constexpr int H = 1 << MH;
-#pragma unroll 1
-    for (int tau = gtid<NT>(); tau < H / 2 + 1; tau += NT) half_pointwise_pair(s2, s1, H, ab2, ab1, tau);
-    gsync<NT>();
+    half_pointwise_all<NT, split_groups<NT, SP>(H / 2)>(s2, s1, H, ab2, ab1);
 }
 
 // half_forward's packing (cpu.rs:286-295): z_j = v_2j + i v_2j+1 for j < h, at swz(j). Ends
@@ -204,39 +221,39 @@ template <int M> constexpr int smem_bytes() { return 24 << M; }
 
 // REDC from T (in tl, 2n limbs) into x (n limbs), wraparound path. Returns false on a carry
 // out that must vanish.
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __noinline__ bool redc_wrap(F2* s2, F1* s1, const uint32_t* tl, uint32_t* x, const F2* cc2, const F1* cc1,
                                           const F2K* tab2, const F1* tab1, uint64_t* sc) {
     constexpr int N = 1 << M;
     const F2K* ht2 = tab2 + lt_half_off(M);
     const F1* ht1 = tab1 + lt_half_off(M);
-    fwd_limbs<M, NT>(tl, N, s2, s1, tab2, tab1);
-    fused_mid<M, NT, true>(tl, N, s2, s1, tab2, tab1, SpecMulOp<M>{cc2, cc1});
-    inv_to_natural<M, NT, true>(s2, s1, tab2, tab1);
+    fwd_limbs<M, NT, SP>(tl, N, s2, s1, tab2, tab1);
+    fused_mid<M, NT, true, SP>(tl, N, s2, s1, tab2, tab1, SpecMulOp<M>{cc2, cc1});
+    inv_to_natural<M, NT, true, SP>(s2, s1, tab2, tab1);
     carry_low_and_pack<M, NT>(s2, s1, sc);
-    dif_unweighted<M - 1, NT>(s2, s1, ht2, ht1);
-    half_pointwise<M - 1, NT>(s2, s1, cc2 + N, cc1 + N);
-    dit_unweighted<M - 1, NT>(s2, s1, ht2, ht1);
+    dif_unweighted<M - 1, NT, SP>(s2, s1, ht2, ht1);
+    half_pointwise<M - 1, NT, SP>(s2, s1, cc2 + N, cc1 + N);
+    dit_unweighted<M - 1, NT, SP>(s2, s1, ht2, ht1);
     return wrap_combine<M, NT>(s2, s1, tl, x, sc);
 }
 
 // REDC without the wraparound path (cpu.rs:453-484 with half = None), k <= n limbs: m = (T mod R)
 // N' mod R through F(N'), then m N through F(N) (both in cc, fused-pass order), and
 // x = T_high + (m N)_high + [T mod R != 0]. m overwrites x, which the step no longer needs.
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __noinline__ bool redc_plain(F2* s2, F1* s1, const uint32_t* tl, uint32_t* x, const F2* cc2, const F1* cc1,
                                         const F2K* tab2, const F1* tab1, uint64_t* sc, int k) {
     constexpr int N = 1 << M;
     int nz = 0;
     for (int q = gtid<NT>(); q < k; q += NT) nz |= tl[q] != 0;
     const uint32_t flag = gsync_or<NT>(nz) ? 1u : 0u;
-    fwd_limbs<M, NT>(tl, k, s2, s1, tab2, tab1);
-    fused_mid<M, NT, true>(tl, k, s2, s1, tab2, tab1, SpecMulOp<M>{cc2, cc1});
-    inv_to_natural<M, NT, true>(s2, s1, tab2, tab1);
+    fwd_limbs<M, NT, SP>(tl, k, s2, s1, tab2, tab1);
+    fused_mid<M, NT, true, SP>(tl, k, s2, s1, tab2, tab1, SpecMulOp<M>{cc2, cc1});
+    inv_to_natural<M, NT, true, SP>(s2, s1, tab2, tab1);
     carry_low_to<M, NT>(s2, s1, x, k, sc);
-    fwd_limbs<M, NT>(x, k, s2, s1, tab2, tab1);
-    fused_mid<M, NT, false>(x, k, s2, s1, tab2, tab1, SpecMulOp<M>{cc2 + N, cc1 + N});
-    inv_to_natural<M, NT, false>(s2, s1, tab2, tab1);
+    fwd_limbs<M, NT, SP>(x, k, s2, s1, tab2, tab1);
+    fused_mid<M, NT, false, SP>(x, k, s2, s1, tab2, tab1, SpecMulOp<M>{cc2 + N, cc1 + N});
+    inv_to_natural<M, NT, false, SP>(s2, s1, tab2, tab1);
     return carry_shift_add<M, NT>(s2, s1, tl, x, k, flag, sc);
 }
 
@@ -244,7 +261,7 @@ __device__ __noinline__ bool redc_plain(F2* s2, F1* s1, const uint32_t* tl, uint
 // vector in `smem_raw` (24 n bytes). Used by the uniform launch and the mixed-length launch.
 // With a.bare each step ends after T = c x^2 and x stays as it was (the reference's run_bare,
 // lib.rs:883-927, which times the squaring alone).
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __forceinline__ void step_slot(const SlotArgs& a, uint32_t slot, uint32_t bits, unsigned char* smem_raw,
                                           uint64_t* sc) {
     constexpr int N = 1 << M;
@@ -262,13 +279,13 @@ __device__ __forceinline__ void step_slot(const SlotArgs& a, uint32_t slot, uint
     for (uint32_t it = 0; it < bits && pos < nb; ++it, ++pos) {
         const uint32_t bit = (ex[pos >> 5] >> (31 - (pos & 31))) & 1;
         const uint32_t c = bit ? a.base : 1;
-        fwd_limbs<M, NT>(x, k, s2, s1, a.tab2, a.tab1);
-        fused_mid<M, NT, false>(x, k, s2, s1, a.tab2, a.tab1, SquareOp{c});
-        inv_to_natural<M, NT, false>(s2, s1, a.tab2, a.tab1);
+        fwd_limbs<M, NT, SP>(x, k, s2, s1, a.tab2, a.tab1);
+        fused_mid<M, NT, false, SP>(x, k, s2, s1, a.tab2, a.tab1, SquareOp{c});
+        inv_to_natural<M, NT, false, SP>(s2, s1, a.tab2, a.tab1);
         ok &= carry_product<M, NT>(s2, s1, tl, sc) == 0;
         if (a.bare) continue;
-        if (a.plain) ok &= redc_plain<M, NT>(s2, s1, tl, x, cc2, cc1, a.tab2, a.tab1, sc, k);
-        else ok &= redc_wrap<M, NT>(s2, s1, tl, x, cc2, cc1, a.tab2, a.tab1, sc);
+        if (a.plain) ok &= redc_plain<M, NT, SP>(s2, s1, tl, x, cc2, cc1, a.tab2, a.tab1, sc, k);
+        else ok &= redc_wrap<M, NT, SP>(s2, s1, tl, x, cc2, cc1, a.tab2, a.tab1, sc);
     }
     gsync<NT>();   // every thread has read pos before it is written
     if (gtid<NT>() == 0) {
@@ -280,16 +297,16 @@ __device__ __forceinline__ void step_slot(const SlotArgs& a, uint32_t slot, uint
 // The uniform launch: one block per slot first + blockIdx.x, `bits` steps each; or, with an item
 // list, one block per item (slot, steps) of the list (a serving tick's launch over the busy slots
 // of a batch; each slot at most once).
-template <int M, int NT, int MINB = (M <= 12 ? 2 : 1)>
+template <int M, int NT, int MINB = (M <= 12 ? 2 : 1), bool SP = false>
 __global__ void __launch_bounds__(NT, MINB)
     step_kernel(SlotArgs a, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<NT>::words];
     if (items) {
         const uint2 it = items[blockIdx.x];
-        step_slot<M, NT>(a, it.x, it.y, smem_raw, sc);
+        step_slot<M, NT, SP>(a, it.x, it.y, smem_raw, sc);
     } else {
-        step_slot<M, NT>(a, first + blockIdx.x, bits, smem_raw, sc);
+        step_slot<M, NT, SP>(a, first + blockIdx.x, bits, smem_raw, sc);
     }
 }
 

@@ -181,73 +181,102 @@ template <> __device__ __forceinline__ void bf_dif<8, F2>(F2* x) { bf_dif8(x); }
 template <> __device__ __forceinline__ void bf_dit<8, F1>(F1* x) { bf_dit8(x); }
 template <> __device__ __forceinline__ void bf_dit<8, F2>(F2* x) { bf_dit8(x); }
 
+// ---- how a pass's groups are spread over the threads ----
+// A group's M61 part and its M31 part touch different arrays. By default each thread does both
+// parts of its groups, one after the other. The wide shapes (template argument SP; at least two
+// threads per group) split a pass: the lower half of the threads does the M61 parts and the upper
+// half the M31 parts, at the same time. That shortens a pass, which is what counts when a batch
+// leaves SMs idle (wide_threads_for, mm_abi.h: L = 512 on 64 slots, 45.9 us a step with one warp per
+// slot, 31 us with two); on a full GPU other warps hide the same latency and the second copy of
+// each pass costs more (L = 8,192's half-length passes split: 617 -> 662 ns per slot-step).
+template <int NT, bool SP> MM_HD constexpr bool split_groups(int G) { return SP && NT >= 64 && 2 * G <= NT; }
+template <int NT, bool SPLIT, class P2, class P1>
+__device__ __forceinline__ void for_groups(int G, const P2& part2, const P1& part1) {
+    if constexpr (SPLIT) {
+        const int t = gtid<NT>() & (NT / 2 - 1);
+        if (gtid<NT>() < NT / 2) {
+#pragma unroll 1
+            for (int g = t; g < G; g += NT / 2) part2(g);
+        } else {
+#pragma unroll 1
+            for (int g = t; g < G; g += NT / 2) part1(g);
+        }
+    } else {
+#pragma unroll 1
+        for (int g = gtid<NT>(); g < G; g += NT) {
+            part2(g);
+            part1(g);
+        }
+    }
+}
+
 // ---- one pass over the shared vector ----
 // A radix-R pass with span q = 2^LQ over G = n/R groups, twiddles `t2`/`t1` laid out
 // [k-1][j] (TW) or none (span 1). One non-inlined function per (R, direction, TW) with a
 // runtime span serves every pass of every transform: the smaller code measured faster than one
 // instance per span, because the step loop's code then stays within the instruction cache.
-template <int R, bool FWD, int NT, bool TW>
+template <int R, bool FWD, int NT, bool TW, bool SPLIT = false>
 __device__ __noinline__ void pass_rt(F2* s2, F1* s1, const F2K* __restrict__ t2, const F1* __restrict__ t1, int LQ, int G) {
     const int q = 1 << LQ;
     // swz(k q) for k < R: swz is linear over XOR, so the offsets are XORs of those of the
     // span's powers of two q, 2q, 4q (three registers instead of R).
     const int kb0 = swz(q), kb1 = R > 2 ? swz(2 * q) : 0, kb2 = R > 4 ? swz(4 * q) : 0;
 #define MM_KO(k) ((((k) & 1) ? kb0 : 0) ^ (((k) & 2) ? kb1 : 0) ^ (((k) & 4) ? kb2 : 0))
-#pragma unroll 1
-    for (int g = gtid<NT>(); g < G; g += NT) {
+    const auto part2 = [&](int g) {
         const int j = g & (q - 1);
         // b + k q has disjoint bits: swz(b + k q) = swz(b) ^ swz(k q).
         const int sb = swz(((g >> LQ) << (LQ + ilog2c(R))) + j);
-        {
-            F2 x[R];
+        F2 x[R];
 #pragma unroll
-            for (int k = 0; k < R; ++k) x[k] = s2[sb ^ MM_KO(k)];
-            if (FWD) {
-                ldif<R>(x);
-                x[0] = lcfold(x[0]);
+        for (int k = 0; k < R; ++k) x[k] = s2[sb ^ MM_KO(k)];
+        if (FWD) {
+            ldif<R>(x);
+            x[0] = lcfold(x[0]);
 #pragma unroll
-                for (int k = 1; k < R; ++k) x[k] = TW ? lkmul(lcfold(x[k]), t2[(k - 1) * q + j]) : lcfold(x[k]);
-            } else {
-                if (TW) {
+            for (int k = 1; k < R; ++k) x[k] = TW ? lkmul(lcfold(x[k]), t2[(k - 1) * q + j]) : lcfold(x[k]);
+        } else {
+            if (TW) {
 #pragma unroll
-                    for (int k = 1; k < R; ++k) x[k] = lkmul(x[k], t2[(k - 1) * q + j]);
-                }
-                ldit<R>(x);
+                for (int k = 1; k < R; ++k) x[k] = lkmul(x[k], t2[(k - 1) * q + j]);
             }
-#pragma unroll
-            for (int k = 0; k < R; ++k) s2[sb ^ MM_KO(k)] = x[k];
+            ldit<R>(x);
         }
-        {
-            F1 x[R];
 #pragma unroll
-            for (int k = 0; k < R; ++k) x[k] = s1[sb ^ MM_KO(k)];
-            if (FWD) {
-                bf_dif<R, F1>(x);
-                if (TW) {
+        for (int k = 0; k < R; ++k) s2[sb ^ MM_KO(k)] = x[k];
+    };
+    const auto part1 = [&](int g) {
+        const int j = g & (q - 1);
+        const int sb = swz(((g >> LQ) << (LQ + ilog2c(R))) + j);
+        F1 x[R];
 #pragma unroll
-                    for (int k = 1; k < R; ++k) x[k] = cmul(x[k], t1[(k - 1) * q + j]);
-                }
-            } else {
-                if (TW) {
+        for (int k = 0; k < R; ++k) x[k] = s1[sb ^ MM_KO(k)];
+        if (FWD) {
+            bf_dif<R, F1>(x);
+            if (TW) {
 #pragma unroll
-                    for (int k = 1; k < R; ++k) x[k] = cmul(x[k], t1[(k - 1) * q + j]);
-                }
-                bf_dit<R, F1>(x);
+                for (int k = 1; k < R; ++k) x[k] = cmul(x[k], t1[(k - 1) * q + j]);
             }
+        } else {
+            if (TW) {
 #pragma unroll
-            for (int k = 0; k < R; ++k) s1[sb ^ MM_KO(k)] = x[k];
+                for (int k = 1; k < R; ++k) x[k] = cmul(x[k], t1[(k - 1) * q + j]);
+            }
+            bf_dit<R, F1>(x);
         }
-    }
+#pragma unroll
+        for (int k = 0; k < R; ++k) s1[sb ^ MM_KO(k)] = x[k];
+    };
+    for_groups<NT, SPLIT>(G, part2, part1);
 #undef MM_KO
     gsync<NT>();
 }
 
 // Pass I (DIF order) of the length-2^M transform; its table follows mm_common.h's layout.
-template <int M, int I, bool FWD, int NT, bool WEIGHTED>
+template <int M, int I, bool FWD, int NT, bool WEIGHTED, bool SP = false>
 __device__ __forceinline__ void smem_pass(F2* s2, F1* s1, const F2K* tab2, const F1* tab1) {
     constexpr int R = sched_radix(M, I), Q = sched_q(M, I);
     constexpr int toff = FWD ? tab_fwd_off(M, I, WEIGHTED) : tab_inv_off(M, I, WEIGHTED);
-    pass_rt<R, FWD, NT, (Q > 1)>(s2, s1, tab2 + toff, tab1 + toff, ilog2c(Q), (1 << M) / R);
+    pass_rt<R, FWD, NT, (Q > 1), split_groups<NT, SP>((1 << M) / R)>(s2, s1, tab2 + toff, tab1 + toff, ilog2c(Q), (1 << M) / R);
 }
 
 // ---- the weighted first DIF pass, straight from real limbs in global memory ----
@@ -261,12 +290,37 @@ template <> __device__ __forceinline__ F1 real_times<F1>(uint32_t v, F1 c) {
     return cmul_r(s, c);
 }
 
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __noinline__ void dif_first_from_limbs(const uint32_t* __restrict__ lim, int cnt, F2* s2, F1* s1,
                                                      const F2K* tab2, const F1* tab1) {
     constexpr int R = sched_radix(M, 0), Q = sched_q(M, 0);
     static_assert(Q > 1, "single-pass transforms use the fused pass");
     constexpr int toff = tab_fwd_off(M, 0, true), coff = tab_in_const_off(M, true);
+    if constexpr (split_groups<NT, SP>(Q)) {
+        const auto limb = [&](int j, int k) { return (j + k * Q < cnt) ? lim[j + k * Q] : 0u; };
+        for_groups<NT, true>(
+            Q,
+            [&](int j) {
+                const int sj = swz(j);   // j < Q: swz(j + k Q) = swz(j) ^ swz(k Q)
+                F2 x[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) x[k] = lreal_times(limb(j, k), tab2[coff + k]);
+                ldif<R>(x);
+#pragma unroll
+                for (int k = 0; k < R; ++k) s2[(sj ^ swz_c(k * Q))] = lkmul(lcfold(x[k]), tab2[toff + k * Q + j]);
+            },
+            [&](int j) {
+                const int sj = swz(j);
+                F1 x[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) x[k] = real_times<F1>(limb(j, k), tab1[coff + k]);
+                bf_dif<R, F1>(x);
+#pragma unroll
+                for (int k = 0; k < R; ++k) s1[(sj ^ swz_c(k * Q))] = cmul(x[k], tab1[toff + k * Q + j]);
+            });
+        gsync<NT>();
+        return;
+    }
 #pragma unroll 1
     for (int j = gtid<NT>(); j < Q; j += NT) {
         const int sj = swz(j);   // j < Q: swz(j + k Q) = swz(j) ^ swz(k Q)
@@ -295,37 +349,36 @@ __device__ __noinline__ void dif_first_from_limbs(const uint32_t* __restrict__ l
 
 // ---- the weighted last DIT pass: unweights by zeta^-(j + k q) / n into natural order ----
 // REAL_ONLY: only the real parts are needed (the low half of the product, coefficients < n).
-template <int M, int NT, bool REAL_ONLY>
+template <int M, int NT, bool REAL_ONLY, bool SP = false>
 __device__ __noinline__ void dit_last_weighted(F2* s2, F1* s1, const F2K* tab2, const F1* tab1) {
     constexpr int R = sched_radix(M, 0), Q = sched_q(M, 0);
     static_assert(Q > 1, "single-pass transforms use the fused pass");
     constexpr int toff = tab_inv_off(M, 0, true), coff = tab_out_const_off(M, true);
-#pragma unroll 1
-    for (int j = gtid<NT>(); j < Q; j += NT) {
+    const auto part2 = [&](int j) {
         const int sj = swz(j);   // j < Q: swz(j + k Q) = swz(j) ^ swz(k Q)
-        {
-            F2 x[R];
+        F2 x[R];
 #pragma unroll
-            for (int k = 0; k < R; ++k) x[k] = lkmul(s2[(sj ^ swz_c(k * Q))], tab2[toff + k * Q + j]);
-            ldit<R>(x);
+        for (int k = 0; k < R; ++k) x[k] = lkmul(s2[(sj ^ swz_c(k * Q))], tab2[toff + k * Q + j]);
+        ldit<R>(x);
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                if (REAL_ONLY) s2[(sj ^ swz_c(k * Q))].re = lkmul_re(x[k], tab2[coff + k]);
-                else s2[(sj ^ swz_c(k * Q))] = lkmul(x[k], tab2[coff + k]);
-            }
+        for (int k = 0; k < R; ++k) {
+            if (REAL_ONLY) s2[(sj ^ swz_c(k * Q))].re = lkmul_re(x[k], tab2[coff + k]);
+            else s2[(sj ^ swz_c(k * Q))] = lkmul(x[k], tab2[coff + k]);
         }
-        {
-            F1 x[R];
+    };
+    const auto part1 = [&](int j) {
+        const int sj = swz(j);
+        F1 x[R];
 #pragma unroll
-            for (int k = 0; k < R; ++k) x[k] = cmul(s1[(sj ^ swz_c(k * Q))], tab1[toff + k * Q + j]);
-            bf_dit<R, F1>(x);
+        for (int k = 0; k < R; ++k) x[k] = cmul(s1[(sj ^ swz_c(k * Q))], tab1[toff + k * Q + j]);
+        bf_dit<R, F1>(x);
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                if (REAL_ONLY) s1[(sj ^ swz_c(k * Q))].re = cmul_re(x[k], tab1[coff + k]);
-                else s1[(sj ^ swz_c(k * Q))] = cmul(x[k], tab1[coff + k]);
-            }
+        for (int k = 0; k < R; ++k) {
+            if (REAL_ONLY) s1[(sj ^ swz_c(k * Q))].re = cmul_re(x[k], tab1[coff + k]);
+            else s1[(sj ^ swz_c(k * Q))] = cmul(x[k], tab1[coff + k]);
         }
-    }
+    };
+    for_groups<NT, split_groups<NT, SP>(Q)>(Q, part2, part1);
     gsync<NT>();
 }
 
@@ -393,7 +446,7 @@ __device__ __noinline__ void dit_last_complex(F2* s2, F1* s1, const F2K* tab2, c
 // ---- the fused middle: last DIF pass (span 1), a pointwise operation, first DIT pass ----
 // OP::apply2/apply1(x, g) transforms the R spectrum values of group g (positions R g + k).
 // With a single pass (M <= 3) the same pass is also the weighted first/last pass.
-template <int M, int NT, bool REAL_ONLY, class OP>
+template <int M, int NT, bool REAL_ONLY, bool SP = false, class OP>
 __device__ __noinline__ void fused_mid(const uint32_t* __restrict__ lim, int cnt, F2* s2, F1* s1,
                                           const F2K* tab2, const F1* tab1, const OP& op) {
     constexpr int P = sched_passes(M);
@@ -401,107 +454,106 @@ __device__ __noinline__ void fused_mid(const uint32_t* __restrict__ lim, int cnt
     constexpr int G = (1 << M) / R;
     constexpr bool single = (P == 1);
     constexpr int cin = tab_in_const_off(M, true), cout = tab_out_const_off(M, true);
-#pragma unroll 1
-    for (int g = gtid<NT>(); g < G; g += NT) {
+    const auto part2 = [&](int g) {
         const int sg = swz(R * g);   // swz(R g + k) = swz(R g) ^ k for k < R <= 8
-        {
-            F2 x[R];
-            if (single) {
+        F2 x[R];
+        if (single) {
 #pragma unroll
-                for (int k = 0; k < R; ++k) x[k] = lreal_times(k < cnt ? lim[k] : 0u, tab2[cin + k]);
-            } else {
+            for (int k = 0; k < R; ++k) x[k] = lreal_times(k < cnt ? lim[k] : 0u, tab2[cin + k]);
+        } else {
 #pragma unroll
-                for (int k = 0; k < R; ++k) x[k] = s2[(sg ^ k)];
-            }
-            ldif<R>(x);
+            for (int k = 0; k < R; ++k) x[k] = s2[(sg ^ k)];
+        }
+        ldif<R>(x);
 #pragma unroll
-            for (int k = 0; k < R; ++k) x[k] = lcfold(x[k]);
-            if (!op.template apply2<R>(x, g)) {
-                ldit<R>(x);
+        for (int k = 0; k < R; ++k) x[k] = lcfold(x[k]);
+        if (!op.template apply2<R>(x, g)) {
+            ldit<R>(x);
 #pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    if (single) {
-                        if (REAL_ONLY) s2[k].re = lkmul_re(x[k], tab2[cout + k]);
-                        else s2[k] = lkmul(x[k], tab2[cout + k]);
-                    } else {
-                        s2[(sg ^ k)] = x[k];
-                    }
+            for (int k = 0; k < R; ++k) {
+                if (single) {
+                    if (REAL_ONLY) s2[k].re = lkmul_re(x[k], tab2[cout + k]);
+                    else s2[k] = lkmul(x[k], tab2[cout + k]);
+                } else {
+                    s2[(sg ^ k)] = x[k];
                 }
             }
         }
-        {
-            F1 x[R];
-            if (single) {
+    };
+    const auto part1 = [&](int g) {
+        const int sg = swz(R * g);
+        F1 x[R];
+        if (single) {
 #pragma unroll
-                for (int k = 0; k < R; ++k) x[k] = real_times<F1>(k < cnt ? lim[k] : 0u, tab1[cin + k]);
-            } else {
+            for (int k = 0; k < R; ++k) x[k] = real_times<F1>(k < cnt ? lim[k] : 0u, tab1[cin + k]);
+        } else {
 #pragma unroll
-                for (int k = 0; k < R; ++k) x[k] = s1[(sg ^ k)];
-            }
-            bf_dif<R, F1>(x);
-            if (!op.template apply1<R>(x, g)) {
-                bf_dit<R, F1>(x);
+            for (int k = 0; k < R; ++k) x[k] = s1[(sg ^ k)];
+        }
+        bf_dif<R, F1>(x);
+        if (!op.template apply1<R>(x, g)) {
+            bf_dit<R, F1>(x);
 #pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    if (single) {
-                        if (REAL_ONLY) s1[k].re = cmul_re(x[k], tab1[cout + k]);
-                        else s1[k] = cmul(x[k], tab1[cout + k]);
-                    } else {
-                        s1[(sg ^ k)] = x[k];
-                    }
+            for (int k = 0; k < R; ++k) {
+                if (single) {
+                    if (REAL_ONLY) s1[k].re = cmul_re(x[k], tab1[cout + k]);
+                    else s1[k] = cmul(x[k], tab1[cout + k]);
+                } else {
+                    s1[(sg ^ k)] = x[k];
                 }
             }
         }
-    }
+    };
+    for_groups<NT, split_groups<NT, SP>(G)>(G, part2, part1);
     gsync<NT>();
 }
 
 // ---- whole transforms ----
 // Forward weighted transform of real limbs up to (not including) the last pass.
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __forceinline__ void fwd_limbs(const uint32_t* __restrict__ lim, int cnt, F2* s2, F1* s1,
                                           const F2K* t2, const F1* t1) {
     constexpr int P = sched_passes(M);
     if constexpr (P >= 2) {
-        dif_first_from_limbs<M, NT>(lim, cnt, s2, s1, t2, t1);
-        if constexpr (P >= 3) smem_pass<M, 1, true, NT, true>(s2, s1, t2, t1);
-        if constexpr (P >= 4) smem_pass<M, 2, true, NT, true>(s2, s1, t2, t1);
-        if constexpr (P >= 5) smem_pass<M, 3, true, NT, true>(s2, s1, t2, t1);
+        dif_first_from_limbs<M, NT, SP>(lim, cnt, s2, s1, t2, t1);
+        if constexpr (P >= 3) smem_pass<M, 1, true, NT, true, SP>(s2, s1, t2, t1);
+        if constexpr (P >= 4) smem_pass<M, 2, true, NT, true, SP>(s2, s1, t2, t1);
+        if constexpr (P >= 5) smem_pass<M, 3, true, NT, true, SP>(s2, s1, t2, t1);
         static_assert(P <= 5, "schedule longer than the shared-memory lengths need");
     }
 }
 
 // Inverse weighted transform from after the fused pass down to natural order.
-template <int M, int NT, bool REAL_ONLY>
+template <int M, int NT, bool REAL_ONLY, bool SP = false>
 __device__ __forceinline__ void inv_to_natural(F2* s2, F1* s1, const F2K* t2, const F1* t1) {
     constexpr int P = sched_passes(M);
     if constexpr (P >= 2) {
-        if constexpr (P >= 5) smem_pass<M, 3, false, NT, true>(s2, s1, t2, t1);
-        if constexpr (P >= 4) smem_pass<M, 2, false, NT, true>(s2, s1, t2, t1);
-        if constexpr (P >= 3) smem_pass<M, 1, false, NT, true>(s2, s1, t2, t1);
-        dit_last_weighted<M, NT, REAL_ONLY>(s2, s1, t2, t1);
+        if constexpr (P >= 5) smem_pass<M, 3, false, NT, true, SP>(s2, s1, t2, t1);
+        if constexpr (P >= 4) smem_pass<M, 2, false, NT, true, SP>(s2, s1, t2, t1);
+        if constexpr (P >= 3) smem_pass<M, 1, false, NT, true, SP>(s2, s1, t2, t1);
+        dit_last_weighted<M, NT, REAL_ONLY, SP>(s2, s1, t2, t1);
     }
 }
 
 // Unweighted transforms of the first 2^M elements (the wraparound path's length h), all in smem.
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __forceinline__ void dif_unweighted(F2* s2, F1* s1, const F2K* t2, const F1* t1) {
     constexpr int P = sched_passes(M);
-    smem_pass<M, 0, true, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 2) smem_pass<M, 1, true, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 3) smem_pass<M, 2, true, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 4) smem_pass<M, 3, true, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 5) smem_pass<M, 4, true, NT, false>(s2, s1, t2, t1);
+    smem_pass<M, 0, true, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 2) smem_pass<M, 1, true, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 3) smem_pass<M, 2, true, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 4) smem_pass<M, 3, true, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 5) smem_pass<M, 4, true, NT, false, SP>(s2, s1, t2, t1);
     static_assert(P <= 5, "schedule longer than the shared-memory lengths need");
 }
-template <int M, int NT>
+template <int M, int NT, bool SP = false>
 __device__ __forceinline__ void dit_unweighted(F2* s2, F1* s1, const F2K* t2, const F1* t1) {
     constexpr int P = sched_passes(M);
-    if constexpr (P >= 5) smem_pass<M, 4, false, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 4) smem_pass<M, 3, false, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 3) smem_pass<M, 2, false, NT, false>(s2, s1, t2, t1);
-    if constexpr (P >= 2) smem_pass<M, 1, false, NT, false>(s2, s1, t2, t1);
-    smem_pass<M, 0, false, NT, false>(s2, s1, t2, t1);
+    if constexpr (P >= 5) smem_pass<M, 4, false, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 4) smem_pass<M, 3, false, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 3) smem_pass<M, 2, false, NT, false, SP>(s2, s1, t2, t1);
+    if constexpr (P >= 2) smem_pass<M, 1, false, NT, false, SP>(s2, s1, t2, t1);
+    smem_pass<M, 0, false, NT, false, SP>(s2, s1, t2, t1);
 }
 
 }  // namespace mm

@@ -1,5 +1,5 @@
-"""The shapes run chooses by itself (no counterpart in the reference): clusters of eight blocks at
-L = 131072. Raw limbs equal those of the same batch stepped another way."""
+"""The shapes run chooses by itself (no counterpart in the reference): wide blocks for batches that
+leave SMs idle, clusters of eight blocks at L = 131072. Raw limbs equal those of the same batch stepped another way."""
 import random
 
 import numpy as np
@@ -30,6 +30,20 @@ def batch(gpu, bits, slots, nbits, base=3, seed=1):
 def raw(b):
     be, st = b.backend_and_state()
     return np.array(be.read_all(st))
+
+
+# Transform lengths with wide shapes (L = 128 to 4096): the top of a bucket, an odd size, and
+# more slots than the widest shape holds at once (which takes the next one).
+@pytest.mark.parametrize("bits,slots", [(16 * (1 << e) - 4, s) for e in range(7, 13) for s in (1, 3)] +
+                         [(1500, 2), (4097, 400), (9001, 300), (33_000, 160)])
+def test_wide_shapes_same_raw_as_default_shape(gpu, bits, slots):
+    nbits = [9 + i % 3 for i in range(slots)]
+    a, b = batch(gpu, bits, slots, nbits), batch(gpu, bits, slots, nbits)
+    be, st = b.backend_and_state()
+    be.set_schedule(st, 0, 0, 0.0, be.get_schedule(st)["threads"])   # a named shape stays
+    a.run(100)
+    b.run(100)
+    assert np.array_equal(raw(a), raw(b))
 
 
 def test_clusters_of_eight_same_raw_as_global_mode(gpu):
