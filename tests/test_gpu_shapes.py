@@ -1,10 +1,12 @@
 """The shapes run chooses by itself (no counterpart in the reference): wide blocks for batches that
-leave SMs idle, clusters of eight blocks at L = 131072. Raw limbs equal those of the same batch stepped another way."""
+leave SMs idle, slots taken in rotation where they do not fill whole waves, clusters of eight blocks
+at L = 131072. Raw limbs equal those of the same batch stepped another way."""
 import random
 
 import numpy as np
 import pytest
 
+import common
 from montmul_b200 import ModBatch
 
 pytestmark = pytest.mark.gpu
@@ -43,6 +45,22 @@ def test_wide_shapes_same_raw_as_default_shape(gpu, bits, slots):
     be.set_schedule(st, 0, 0, 0.0, be.get_schedule(st)["threads"])   # a named shape stays
     a.run(100)
     b.run(100)
+    assert np.array_equal(raw(a), raw(b))
+
+
+# L = 16384 holds one slot per SM, L = 32768 and 65536 a cluster per 2 and 4 SMs: a few slots
+# more than fit, with exponents that end at different steps, in one run and step by step (which
+# does not rotate).
+@pytest.mark.parametrize("bits,slots,steps", [(200_000, 150, 24), (500_000, 77, 12), (1_000_000, 38, 12)])
+def test_rotation_same_raw_as_single_steps(gpu, bits, slots, steps):
+    nbits = [steps if i % 5 else 1 + i % steps for i in range(slots)]
+    a, b = batch(gpu, bits, slots, nbits, base=2), batch(gpu, bits, slots, nbits, base=2)
+    be, st = a.backend_and_state()
+    before = be.launches(st)
+    a.run(steps)
+    assert be.launches(st) - before > 1 and all(a.remaining(i) == 0 for i in range(slots))
+    for _ in range(steps):
+        b.run(1)
     assert np.array_equal(raw(a), raw(b))
 
 
