@@ -181,8 +181,9 @@ __device__ __forceinline__ void half_factors_block(F2* s2, F1* s1, int H, const 
 }
 
 // The Transform trait's forward (weight by zeta^j, DIF) or inverse (DIT, unweight by
-// zeta^-j / n) of vector first + blockIdx.x, in place in a device buffer whose element order is
-// the kernels' (element j at swz(j)); the result is canonical (cpu.rs:86-103, 349-407).
+// zeta^-j / n) of vector first + blockIdx.x, in place in a device buffer in natural element order
+// (swz, which permutes within 16 elements, applies on the way into and out of shared memory); the
+// result is canonical (cpu.rs:86-103, 349-407).
 template <int M, int NT>
 __global__ void __launch_bounds__(NT) transform_kernel(F2* v2, F1* v1, const F2K* tab2, const F1* tab1, uint32_t first,
                                                        int inverse) {
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(NT) transform_kernel(F2* v2, F1* v1, const F2K
     F2* g2 = v2 + (size_t)(first + blockIdx.x) * N;
     F1* g1 = v1 + (size_t)(first + blockIdx.x) * N;
     for (int e = gtid<NT>(); e < N; e += NT) {
-        s2[e] = g2[e];
-        s1[e] = g1[e];
+        s2[swz(e)] = g2[e];
+        s1[swz(e)] = g1[e];
     }
     gsync<NT>();
     if (!inverse) {
@@ -211,8 +212,8 @@ __global__ void __launch_bounds__(NT) transform_kernel(F2* v2, F1* v1, const F2K
         dit_last_complex<M, NT>(s2, s1, tab2, tab1);
     }
     for (int e = gtid<NT>(); e < N; e += NT) {
-        g2[e] = lccanon(s2[e]);
-        g1[e] = s1[e];
+        g2[e] = lccanon(s2[swz(e)]);
+        g1[e] = s1[swz(e)];
     }
 }
 
