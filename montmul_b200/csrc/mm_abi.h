@@ -46,6 +46,7 @@ struct KernelSet {
     int threads_alt;
     WideShape wide[kWideShapes];
     MulFn mul;
+    int mul_threads;
     SetupFn setup;
     TransformFn transform;   // the Transform trait's forward / inverse (shared memory)
     int threads;   // block size

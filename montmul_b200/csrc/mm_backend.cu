@@ -930,13 +930,12 @@ int mm_b200_mul(mm_b200_batch* b, size_t out, size_t a, size_t bb) {
         b->gk.mul<<<1, b->gk.threads, b->gk.smem, b->stream>>>(global_args(b), (uint32_t)out, (uint32_t)a, (uint32_t)bb,
                                                               b->d_spec2, b->d_spec1);
     else
-        b->ks.mul<<<1, b->ks.threads, b->ks.smem, b->stream>>>(slot_args(b), (uint32_t)out, (uint32_t)a, (uint32_t)bb,
+        b->ks.mul<<<1, b->ks.mul_threads, b->ks.smem, b->stream>>>(slot_args(b), (uint32_t)out, (uint32_t)a, (uint32_t)bb,
                                                               b->d_spec2, b->d_spec1);
     MM_CK(cudaGetLastError());
     ++b->launches;
-    MM_CK(cudaStreamSynchronize(b->stream));
     b->host_x_valid = false;
-    return check_err(b, "mul");
+    return check_err(b, "mul");   // waits for the stream
 }
 
 int mm_b200_run_items_async(mm_b200_batch* b, size_t count, const size_t* slots, const uint32_t* steps) {

@@ -32,8 +32,9 @@ struct WideStep<M, 0> {
 KernelSet MM_CAT(kernels_m, MM_M)() {
     constexpr int NT = threads_for(MM_M), NTA = alt_threads_for(MM_M);
     constexpr int W0 = wide_threads_for(MM_M, 0), W1 = wide_threads_for(MM_M, 1);
+    constexpr int NTM = W0 ? W0 : W1 ? W1 : NT;   // mul: one block, the widest shape
     return KernelSet{step_kernel<MM_M, NT>, AltStep<MM_M, NTA>::fn(), NTA,
-                     {{WideStep<MM_M, W0>::fn(), W0}, {WideStep<MM_M, W1>::fn(), W1}}, mul_kernel<MM_M, NT>, setup_kernel<MM_M, NT>,
+                     {{WideStep<MM_M, W0>::fn(), W0}, {WideStep<MM_M, W1>::fn(), W1}}, mul_kernel<MM_M, NTM, (NTM != NT)>, NTM, setup_kernel<MM_M, NT>,
                      transform_kernel<MM_M, NT>, NT,
                      smem_bytes<MM_M>()};
 }
