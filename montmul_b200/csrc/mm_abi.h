@@ -27,7 +27,7 @@ struct SlotArgs {
     uint32_t plain;       // 1: REDC without the wraparound path (constants F(N') | F(N))
 };
 
-typedef void (*StepFn)(SlotArgs, uint32_t, uint32_t, const uint2*);
+typedef void (*StepFn)(SlotArgs, StepRange, const uint2*);
 typedef void (*MulFn)(SlotArgs, uint32_t, uint32_t, uint32_t, F2*, F1*);
 typedef void (*SetupFn)(const uint32_t*, const uint32_t*, F2*, F1*, const F2K*, const F1*, F2, F1, uint32_t,
                         const uint32_t*, uint32_t, int);
@@ -61,7 +61,7 @@ struct GArgs {
     F1* w1;
     int m;    // log2 n
 };
-typedef void (*GStepFn)(GArgs, uint32_t, uint32_t, const uint2*);
+typedef void (*GStepFn)(GArgs, StepRange);
 typedef void (*GMulFn)(GArgs, uint32_t, uint32_t, uint32_t, F2*, F1*);
 typedef void (*GSetupFn)(GArgs, const uint32_t*, const uint32_t*, F2*, F1*, F2, F1, uint32_t, const uint32_t*);   // k, plain in g.a
 struct GlobalKernels {
@@ -85,8 +85,8 @@ constexpr int kClusterPairChunkLog = 12;    // the two-blocks-per-SM chunk, at L
 // wraparound batches in global mode (mm_backend.cu).
 constexpr int kClusterWideLogN = 16;
 int cluster_configure();
-// One cluster per slot, `bits` steps each; with items, one per item (slot, steps).
-int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, void* stream);
+// One cluster per slot of the range, `count` of them.
+int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t count, const StepRange& r, void* stream);
 int cluster_capacity(int m, int chunk_log, int* clusters);   // clusters resident at once
 // Enqueues wait_check_kernel (mm_global.cuh) on a stream; non-zero if the launch failed.
 int launch_wait_check(uint32_t* err, uint64_t limit_ns, void* stream);   // mm_global.cu

@@ -15,6 +15,7 @@
 #include "../../include/montmul_b200.h"
 #include "mm_host.hpp"
 #include "mm_abi.h"
+#include "mm_rotation.hpp"
 
 using namespace mm;
 
@@ -134,10 +135,6 @@ struct mm_b200_batch {
     uint2* d_items = nullptr;          // run_items: the list on the device and its pinned staging
     uint2* h_items = nullptr;
     cudaEvent_t items_copied = nullptr;   // the staging may be rewritten once this has passed
-    uint2* d_rot = nullptr;            // run's rotation: its items on the device and their pinned staging
-    uint2* h_rot = nullptr;
-    size_t rot_cap = 0;
-    cudaEvent_t rot_copied = nullptr;
 };
 
 namespace {
@@ -373,82 +370,6 @@ int resident_slots(mm_b200_batch* b, bool clustered, StepFn fn, int threads, siz
     return MM_OK;
 }
 
-// The steps per launch with which `slots` slots of which `resident` fit the device at once finish
-// `steps` steps soonest when launches take the slots in rotation, `resident` at a time; 0 where one
-// launch over all slots is as good. That launch takes ceil(slots / resident) whole waves, the last
-// one of which may leave most SMs idle (37 clusters of L = 65536 where 36 fit: two waves for the
-// work of one); in rotation the idle places go to the next round's slots and only the last launch
-// is partly empty. A launch costs launch_us beyond its steps (its start, and the wait for its slowest
-// block), so a chunk is no shorter than pays for that: 13 us measured for clusters (one block per
-// SM), about 90 us in shared memory, where an SM's blocks finish at different times.
-size_t rotation_chunk(size_t slots, size_t resident, size_t steps, size_t most, double step_us, double launch_us) {
-    if (slots <= resident || slots % resident == 0 || slots > 16 * resident) return 0;
-    double best = 0.97 * (double)((slots + resident - 1) / resident) * (double)steps * step_us;
-    size_t chunk = 0;
-    for (size_t r = 1; r <= 64 && r <= steps; ++r) {
-        const size_t s = (steps + r - 1) / r, rounds = (steps + s - 1) / s;
-        if (s > most) continue;
-        const size_t launches = (slots * rounds + resident - 1) / resident;
-        const double us = (double)launches * ((double)s * step_us + launch_us);
-        if (us < best) {
-            best = us;
-            chunk = s;
-        }
-    }
-    return chunk;
-}
-
-// The launches of a rotation: items (slot, steps) in launch order and the end of each launch's. A
-// slot is listed at most once per launch: a round lists every slot with steps left once, in order,
-// and a launch spans two rounds only while a round still fills a launch.
-void rotation_items(const mm_b200_batch* b, size_t bits, size_t resident, size_t chunk, std::vector<uint2>* items,
-                    std::vector<size_t>* ends) {
-    std::vector<uint32_t> left(b->slots), live;
-    for (size_t i = 0; i < b->slots; ++i) {
-        left[i] = (uint32_t)std::min<size_t>(bits, b->nbits[i] - b->pos[i]);
-        if (left[i]) live.push_back((uint32_t)i);
-    }
-    size_t start = 0;
-    const auto close = [&] {
-        if (items->size() > start) ends->push_back(items->size());
-        start = items->size();
-    };
-    while (!live.empty()) {
-        if (live.size() < resident) close();
-        size_t keep = 0;
-        for (const uint32_t i : live) {
-            const uint32_t s = (uint32_t)std::min<size_t>(chunk, left[i]);
-            items->push_back(make_uint2(i, s));
-            left[i] -= s;
-            if (left[i]) live[keep++] = i;
-            if (items->size() - start == resident) close();
-        }
-        live.resize(keep);
-    }
-    close();
-}
-
-// Uploads the items of a rotation; the previous list may still be read by launches on the stream.
-int upload_items(mm_b200_batch* b, const std::vector<uint2>& items) {
-    if (!b->rot_copied) MM_CK(cudaEventCreateWithFlags(&b->rot_copied, cudaEventDisableTiming));
-    else MM_CK(cudaEventSynchronize(b->rot_copied));
-    if (items.size() > b->rot_cap) {
-        MM_CK(cudaStreamSynchronize(b->stream));
-        if (b->d_rot) MM_CK(cudaFree(b->d_rot));
-        if (b->h_rot) MM_CK(cudaFreeHost(b->h_rot));
-        b->d_rot = nullptr;
-        b->h_rot = nullptr;
-        b->rot_cap = 0;
-        MM_CK(cudaMalloc(&b->d_rot, items.size() * sizeof(uint2)));
-        MM_CK(cudaMallocHost(&b->h_rot, items.size() * sizeof(uint2)));
-        b->rot_cap = items.size();
-    }
-    std::memcpy(b->h_rot, items.data(), items.size() * sizeof(uint2));
-    MM_CK(cudaMemcpyAsync(b->d_rot, b->h_rot, items.size() * sizeof(uint2), cudaMemcpyHostToDevice, b->stream));
-    MM_CK(cudaEventRecord(b->rot_copied, b->stream));
-    return MM_OK;
-}
-
 int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     size_t most = 0, active = 0;
     for (size_t i = 0; i < b->slots; ++i) {
@@ -482,22 +403,19 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         rc = step_shape(b, active, &step_fn, &step_threads);
         if (rc) return rc;
     }
-    // One launch over `count` slots from 0 on, `steps` each, or over `count` items.
-    const auto launch = [&](size_t count, uint32_t steps, const uint2* items) -> int {
+    // One launch over the first `count` slots of a range.
+    const auto launch = [&](size_t count, const StepRange& r) -> int {
         if (clustered) {
-            const int e = cluster_launch(b->m, b->cluster_chunk_log, c, (uint32_t)count, steps, items, b->stream);
+            const int e = cluster_launch(b->m, b->cluster_chunk_log, c, (uint32_t)count, r, b->stream);
             if (e) return fail(MM_ERR_CUDA, std::string("cluster launch: ") + cudaGetErrorString((cudaError_t)e));
         } else if (b->global) {
-            b->gk.step<<<(unsigned)count, b->gk.threads, b->gk.smem, b->stream>>>(g, 0, steps, items);
+            b->gk.step<<<(unsigned)count, b->gk.threads, b->gk.smem, b->stream>>>(g, r);
         } else {
-            step_fn<<<(unsigned)count, step_threads, b->ks.smem, b->stream>>>(a, 0, steps, items);
+            step_fn<<<(unsigned)count, step_threads, b->ks.smem, b->stream>>>(a, r, nullptr);
         }
         MM_CK(cudaGetLastError());
         ++b->launches;
         return MM_OK;
-    };
-    const auto advance = [&](size_t steps) {
-        for (size_t i = 0; i < b->slots; ++i) b->pos[i] += (uint32_t)std::min<size_t>(steps, b->nbits[i] - b->pos[i]);
     };
     const size_t chunk = (size_t)std::max(1, b->sched.launch_steps > 0 ? b->sched.launch_steps : b->dev->max_launch_steps);
     size_t resident = 0;
@@ -507,27 +425,14 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     // times their number, else a model of the transform work.
     const double step_us = b->sched.step_ns > 0 ? 1e-3 * b->sched.step_ns * (double)resident : 1e-3 * (double)b->n * b->m;
     const size_t turn = rotation_chunk(active, resident, left, chunk, step_us, b->global ? 13.0 : 90.0);
-    if (turn) {
-        std::vector<uint2> items;
-        std::vector<size_t> ends;
-        rotation_items(b, left, resident, turn, &items, &ends);
-        rc = upload_items(b, items);
+    // Without a rotation each launch takes every slot once.
+    Rotation rot(b->slots, turn ? resident : b->slots, left, turn ? turn : std::min(left, chunk));
+    StepRange r;
+    size_t count = 0;
+    while (rot.next(b->pos.data(), b->nbits.data(), &r, &count)) {
+        rc = launch(count, r);
         if (rc) return rc;
-        size_t start = 0;
-        for (const size_t end : ends) {
-            rc = launch(end - start, 0, b->d_rot + start);
-            if (rc) return rc;
-            start = end;
-        }
-        advance(left);
-        left = 0;
-    }
-    while (left > 0) {
-        const uint32_t s = (uint32_t)std::min(left, chunk);
-        rc = launch(b->slots, s, nullptr);
-        if (rc) return rc;
-        advance(s);
-        left -= s;
+        rot.advance(r, count, b->pos.data(), b->nbits.data());
     }
     if (!bare) b->host_x_valid = false;
     return MM_OK;
@@ -966,7 +871,7 @@ int mm_b200_run_items_async(mm_b200_batch* b, size_t count, const size_t* slots,
     SlotArgs a = slot_args(b);
     for (size_t first = 0; first < count; first += 65535) {
         const unsigned grid = (unsigned)std::min<size_t>(65535, count - first);
-        b->step_fn<<<grid, b->step_threads, b->ks.smem, b->stream>>>(a, 0, 0, b->d_items + first);
+        b->step_fn<<<grid, b->step_threads, b->ks.smem, b->stream>>>(a, StepRange{}, b->d_items + first);
         MM_CK(cudaGetLastError());
         ++b->launches;
     }
@@ -1054,9 +959,6 @@ void mm_b200_destroy(mm_b200_batch* b) {
     if (b->d_items) cudaFree(b->d_items);
     if (b->h_items) cudaFreeHost(b->h_items);
     if (b->items_copied) cudaEventDestroy(b->items_copied);
-    if (b->d_rot) cudaFree(b->d_rot);
-    if (b->h_rot) cudaFreeHost(b->h_rot);
-    if (b->rot_copied) cudaEventDestroy(b->rot_copied);
     delete b;
 }
 

@@ -18,14 +18,14 @@ int cluster_configure() {
     return (int)e;
 }
 
-int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, void* stream) {
+int cluster_launch(int m, int chunk_log, const SlotArgs& a, uint32_t count, const StepRange& r, void* stream) {
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (chunk_log == kChunkLog) {
-        if (m == 14) return (int)launch_cluster_m<14, kChunkLog>(a, slots, bits, items, s);
-        if (m == 15) return (int)launch_cluster_m<15, kChunkLog>(a, slots, bits, items, s);
-        if (m == 16) return (int)launch_cluster_m<16, kChunkLog>(a, slots, bits, items, s);
+        if (m == 14) return (int)launch_cluster_m<14, kChunkLog>(a, count, r, s);
+        if (m == 15) return (int)launch_cluster_m<15, kChunkLog>(a, count, r, s);
+        if (m == 16) return (int)launch_cluster_m<16, kChunkLog>(a, count, r, s);
     } else if (chunk_log == kClusterPairChunkLog && m == 14) {
-        return (int)cluster_half_chunk_launch(a, slots, bits, items, s);
+        return (int)cluster_half_chunk_launch(a, count, r, s);
     }
     return (int)cudaErrorInvalidValue;
 }

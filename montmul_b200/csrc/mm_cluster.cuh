@@ -531,22 +531,18 @@ __device__ __forceinline__ void cl_step_slot(const SlotArgs& a, uint32_t slot, u
 }
 
 // The uniform cluster launch: cluster i (C = 2^(M - CL) consecutive blocks of 2^CL elements)
-// steps slot first + i, or with an item list item i's (slot, steps). CL = 13: one block of 192 KiB per SM; CL = 12 (L = 32768 only): two
+// steps slot i of the range. CL = 13: one block of 192 KiB per SM; CL = 12 (L = 32768 only): two
 // blocks of 96 KiB per SM, so twice the warps hide the latency of the cross-block accesses, at
 // 64 registers per thread and with more of each cross-block pass remote.
 template <int M, int CL>
 __global__ void __launch_bounds__(kClusterThreads, kChunkLog - CL + 1)
-    cluster_step_kernel(SlotArgs a, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
+    cluster_step_kernel(SlotArgs a, StepRange r) {
     constexpr int C = 1 << (M - CL);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<kClusterThreads>::words];
     __shared__ ClusterCarry cc;
-    uint32_t slot = first + blockIdx.x / C;
-    if (items) {
-        const uint2 it = items[blockIdx.x / C];
-        slot = it.x;
-        bits = it.y;
-    }
+    uint32_t bits;
+    const uint32_t slot = range_slot(r, blockIdx.x / C, bits);
     cl_step_slot<M, kClusterThreads, C>(a, slot, bits, smem_raw, sc, &cc);
 }
 
@@ -569,9 +565,9 @@ struct ClusterLaunch {
 };
 
 template <int M, int CL>
-cudaError_t launch_cluster_m(const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, cudaStream_t s) {
-    const ClusterLaunch l(1 << (M - CL), slots, 24 << CL, s);
-    return cudaLaunchKernelEx(&l.cfg, cluster_step_kernel<M, CL>, a, 0u, bits, items);
+cudaError_t launch_cluster_m(const SlotArgs& a, uint32_t count, const StepRange& r, cudaStream_t s) {
+    const ClusterLaunch l(1 << (M - CL), count, 24 << CL, s);
+    return cudaLaunchKernelEx(&l.cfg, cluster_step_kernel<M, CL>, a, r);
 }
 
 // Clusters the current device holds at once.
@@ -589,7 +585,7 @@ cudaError_t configure_cluster_m() {
 
 // The 4,096-element-chunk instantiation at L = 32768 (mm_cluster_half.cu).
 cudaError_t cluster_half_chunk_configure();
-cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, cudaStream_t s);
+cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t count, const StepRange& r, cudaStream_t s);
 cudaError_t cluster_half_chunk_capacity(int* clusters);
 
 }  // namespace mm

@@ -8,8 +8,8 @@ namespace mm {
 
 cudaError_t cluster_half_chunk_configure() { return configure_cluster_m<14, kClusterPairChunkLog>(); }
 
-cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t slots, uint32_t bits, const uint2* items, cudaStream_t s) {
-    return launch_cluster_m<14, kClusterPairChunkLog>(a, slots, bits, items, s);
+cudaError_t cluster_half_chunk_launch(const SlotArgs& a, uint32_t count, const StepRange& r, cudaStream_t s) {
+    return launch_cluster_m<14, kClusterPairChunkLog>(a, count, r, s);
 }
 
 cudaError_t cluster_half_chunk_capacity(int* clusters) { return capacity_cluster_m<14, kClusterPairChunkLog>(clusters); }

@@ -167,4 +167,17 @@ MM_HD int glt_half_off(int m) { return glt_tile_off(m) + tab_size(kTileLog, fals
 MM_HD int glt_unpack_off(int m) { return glt_half_off(m) + (m - 1 > kTileLog ? gl_tab_size(m - 1, false) : 0); }
 MM_HD int glt_size(int m) { return glt_unpack_off(m) + 2 * (1 << (m - 1)); }
 
+// ---- launches of run ----
+// The slots of one launch of run: block (or cluster) i steps slot first + i, `bits` steps, and past the
+// last of `slots` slots goes on at slot 0 with `bits_next` steps (a launch of a rotation that ends one
+// round and begins the next, mm_rotation.hpp).
+struct StepRange {
+    uint32_t first, slots, bits, bits_next;
+};
+MM_HD uint32_t range_slot(const StepRange& r, uint32_t i, uint32_t& bits) {
+    const uint32_t slot = r.first + i;
+    bits = slot < r.slots ? r.bits : r.bits_next;
+    return slot < r.slots ? slot : slot - r.slots;
+}
+
 }  // namespace mm

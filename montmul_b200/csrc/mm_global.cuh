@@ -617,21 +617,17 @@ __device__ __forceinline__ bool gstep_slot(const GArgs& g, uint32_t slot, uint32
     return st != kStepTimeout;
 }
 
-// The uniform launch, global mode: one block per slot first + blockIdx.x, or per item (slot, steps).
+// The uniform launch, global mode: one block per slot of the range.
 template <int NT>
-__global__ void __launch_bounds__(NT, 2) gstep_kernel(GArgs g, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
+__global__ void __launch_bounds__(NT, 2) gstep_kernel(GArgs g, StepRange r) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<NT>::words];
     __shared__ uint64_t bars[2];
     const TileSmem sm{smem_raw, bars};
     tile_init<NT>(sm);
     uint32_t par = 0;
-    uint32_t slot = first + blockIdx.x;
-    if (items) {
-        const uint2 it = items[blockIdx.x];
-        slot = it.x;
-        bits = it.y;
-    }
+    uint32_t bits;
+    const uint32_t slot = range_slot(r, blockIdx.x, bits);
     gstep_slot<NT>(g, slot, bits, sm, sc, par);
 }
 

@@ -295,19 +295,21 @@ __device__ __forceinline__ void step_slot(const SlotArgs& a, uint32_t slot, uint
     }
 }
 
-// The uniform launch: one block per slot first + blockIdx.x, `bits` steps each; or, with an item
+// The uniform launch: one block per slot of the range; or, with an item
 // list, one block per item (slot, steps) of the list (a serving tick's launch over the busy slots
 // of a batch; each slot at most once).
 template <int M, int NT, int MINB = (M <= 12 ? 2 : 1), bool SP = false>
 __global__ void __launch_bounds__(NT, MINB)
-    step_kernel(SlotArgs a, uint32_t first, uint32_t bits, const uint2* __restrict__ items) {
+    step_kernel(SlotArgs a, StepRange r, const uint2* __restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<NT>::words];
     if (items) {
         const uint2 it = items[blockIdx.x];
         step_slot<M, NT, SP>(a, it.x, it.y, smem_raw, sc);
     } else {
-        step_slot<M, NT, SP>(a, first + blockIdx.x, bits, smem_raw, sc);
+        uint32_t bits;
+        const uint32_t slot = range_slot(r, blockIdx.x, bits);
+        step_slot<M, NT, SP>(a, slot, bits, smem_raw, sc);
     }
 }
 

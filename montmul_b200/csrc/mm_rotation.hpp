@@ -1,0 +1,89 @@
+// How run splits its steps into launches (host code): one launch over all slots, or launches that take
+// the slots in rotation. A rotation needs no list on the device: round r gives every slot the steps
+// from r `chunk` on, the launches cut the sequence of rounds into runs of consecutive slots, and
+// each run is a StepRange in the launch's arguments.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+
+#include "mm_common.h"
+
+namespace mm {
+
+// The steps per launch with which `slots` slots of which `resident` fit the device at once finish
+// `steps` steps soonest when launches take the slots in rotation, `resident` at a time; 0 where one
+// launch over all slots is as good. That launch takes ceil(slots / resident) whole waves, the last
+// one of which may leave most SMs idle (37 clusters of L = 65536 where 36 fit: two waves for the
+// work of one); in rotation the idle places go to the next round's slots and only the last launch
+// is partly empty. A launch costs launch_us beyond its steps (its start, and the wait for its slowest
+// block), so a chunk is no shorter than pays for that: 13 us measured for clusters (one block per
+// SM), about 90 us in shared memory, where an SM's blocks finish at different times.
+inline size_t rotation_chunk(size_t slots, size_t resident, size_t steps, size_t most, double step_us, double launch_us) {
+    if (slots <= resident || slots % resident == 0 || slots > 16 * resident) return 0;
+    double best = 0.97 * (double)((slots + resident - 1) / resident) * (double)steps * step_us;
+    size_t chunk = 0;
+    for (size_t r = 1; r <= 64 && r <= steps; ++r) {
+        const size_t s = (steps + r - 1) / r, rounds = (steps + s - 1) / s;
+        if (s > most) continue;
+        const size_t launches = (slots * rounds + resident - 1) / resident;
+        const double us = (double)launches * ((double)s * step_us + launch_us);
+        if (us < best) {
+            best = us;
+            chunk = s;
+        }
+    }
+    return chunk;
+}
+
+// The launches of one run: `steps` steps on each of `slots` slots (fewer where its exponent ends),
+// `chunk` per launch, in launches of at most `resident` slots with steps left. Slots without steps
+// left are passed over: as blocks that return at once, and not counted. A launch covers at most
+// `slots` consecutive slots, so no slot is in a launch twice.
+class Rotation {
+  public:
+    Rotation(size_t slots, size_t resident, size_t steps, size_t chunk)
+        : slots_(slots), resident_(resident), steps_(steps), chunk_(chunk) {}
+
+    // The next launch that has a slot with steps left; false after the last one. pos and nbits:
+    // per slot, the steps done (advance keeps pos) and the exponent's length.
+    bool next(const uint32_t* pos, const uint32_t* nbits, StepRange* r, size_t* count) {
+        while (round_ * chunk_ < steps_) {
+            size_t n = 0, live = 0, at = slot_, round = round_;
+            while (n < slots_ && live < resident_ && round * chunk_ < steps_) {
+                live += pos[at] < nbits[at];
+                ++n;
+                if (++at == slots_) {
+                    at = 0;
+                    ++round;
+                }
+            }
+            *r = StepRange{(uint32_t)slot_, (uint32_t)slots_, bits(round_), bits(round_ + 1)};
+            *count = n;
+            slot_ = at;
+            round_ = round;
+            if (live) return true;
+        }
+        return false;
+    }
+
+    // What the launch does to pos.
+    static void advance(const StepRange& r, size_t count, uint32_t* pos, const uint32_t* nbits) {
+        for (size_t i = 0; i < count; ++i) {
+            uint32_t bits;
+            const uint32_t s = range_slot(r, (uint32_t)i, bits);
+            pos[s] += std::min(bits, nbits[s] - pos[s]);
+        }
+    }
+
+  private:
+    uint32_t bits(size_t round) const {
+        const size_t done = round * chunk_;
+        return (uint32_t)(done < steps_ ? std::min(chunk_, steps_ - done) : 0);
+    }
+
+    size_t slots_, resident_, steps_, chunk_;
+    size_t slot_ = 0, round_ = 0;   // where the next launch begins
+};
+
+}  // namespace mm

@@ -74,3 +74,25 @@ def test_clusters_of_eight_same_raw_as_global_mode(gpu):
         plan.run(6)
         plan.close()
         assert a.params.len == 131072 and np.array_equal(raw(a), raw(b))
+
+
+def test_queued_runs_in_rotation_do_not_wait_on_the_host(gpu):
+    """run_async returns at once however many runs are queued behind each other, in rotation too."""
+    import time
+    slots, steps = 150, 60
+    b = batch(gpu, 200_000, slots, [6 * steps] * slots, base=2)
+    be, st = b.backend_and_state()
+    be.run_async(st, steps)   # uploads the exponents
+    be.sync(st)
+    t = time.perf_counter()
+    be.run_async(st, steps)
+    be.sync(st)
+    one = time.perf_counter() - t
+    before = be.launches(st)
+    t = time.perf_counter()
+    for _ in range(4):
+        be.run_async(st, steps)
+    host = time.perf_counter() - t
+    assert be.launches(st) - before > 4
+    be.sync(st)
+    assert host < 0.5 * one, (host, one)

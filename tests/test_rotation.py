@@ -1,0 +1,98 @@
+"""How run splits its steps into launches (montmul_b200/csrc/mm_rotation.hpp, built for the host with
+g++): every slot gets the steps it has left, no more than the device holds are stepped at once, and
+no slot is in a launch twice, for any slot counts and exponents. CPU only."""
+import os
+import random
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "montmul_b200", "csrc")
+SOURCE = r'''
+#include "mm_rotation.hpp"
+#include <cstdio>
+#include <cstring>
+#include <vector>
+// "split slots resident steps chunk pos... nbits...": one line per launch, "first bits bits_next: slot/steps ...".
+// "chunk slots resident steps most step_us launch_us": the rotation's steps per launch.
+int main() {
+    char what[16];
+    size_t slots, resident, steps, last;
+    while (std::scanf("%15s %zu %zu %zu %zu", what, &slots, &resident, &steps, &last) == 5) {
+        if (!std::strcmp(what, "chunk")) {
+            double step_us, launch_us;
+            if (std::scanf("%lf %lf", &step_us, &launch_us) != 2) return 1;
+            std::printf("%zu\n", mm::rotation_chunk(slots, resident, steps, last, step_us, launch_us));
+            continue;
+        }
+        std::vector<uint32_t> pos(slots), nbits(slots);
+        for (auto& v : pos) if (std::scanf("%u", &v) != 1) return 1;
+        for (auto& v : nbits) if (std::scanf("%u", &v) != 1) return 1;
+        mm::Rotation rot(slots, resident, steps, last);
+        mm::StepRange r;
+        size_t count;
+        while (rot.next(pos.data(), nbits.data(), &r, &count)) {
+            std::printf("%u %u %u:", r.first, r.bits, r.bits_next);
+            for (uint32_t i = 0; i < count; ++i) {
+                uint32_t bits;
+                const uint32_t s = mm::range_slot(r, i, bits);
+                std::printf(" %u/%u", s, bits);
+            }
+            std::printf("\n");
+            rot.advance(r, count, pos.data(), nbits.data());
+        }
+        std::printf("end");
+        for (auto v : pos) std::printf(" %u", v);
+        std::printf("\n");
+    }
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def ask(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    d = tmp_path_factory.mktemp("rotation")
+    (d / "r.cpp").write_text(SOURCE)
+    subprocess.run([gxx, "-std=c++17", "-I", CSRC, str(d / "r.cpp"), "-o", str(d / "r")], check=True)
+    return lambda q: subprocess.run([str(d / "r")], input=q, check=True, capture_output=True, text=True).stdout.splitlines()
+
+
+def cases(n=400):
+    rng = random.Random(5)
+    for i in range(n):
+        slots = rng.randint(1, 40)
+        steps = rng.randint(1, 50)
+        nbits = [rng.choice([0, 1, steps, rng.randint(0, 60)]) if i % 3 else steps for _ in range(slots)]
+        pos = [rng.randint(0, b) if i % 2 else 0 for b in nbits]
+        yield slots, rng.choice([slots, rng.randint(1, slots)]), steps, rng.randint(1, steps), pos, nbits
+
+
+def test_every_slot_gets_its_steps(ask):
+    all_cases = list(cases())
+    out = iter(ask("\n".join("split " + " ".join(map(str, [*c[:4], *c[4], *c[5]])) for c in all_cases)))
+    for slots, resident, steps, chunk, pos, nbits in all_cases:
+        at = list(pos)
+        for line in out:
+            if line.startswith("end"):
+                break
+            items = [tuple(map(int, w.split("/"))) for w in line.split(":")[1].split()]
+            assert len({s for s, _ in items}) == len(items) <= slots and all(0 <= s < slots for s, _ in items)
+            live = [s for s, _ in items if at[s] < nbits[s]]
+            assert 0 < len(live) <= resident and all(b <= chunk for _, b in items)
+            for s, b in items:
+                at[s] = min(nbits[s], at[s] + b)
+        want = [min(b, p + steps) for p, b in zip(pos, nbits)]
+        assert at == want == [int(v) for v in line.split()[1:]]
+
+
+def test_full_launches_while_enough_slots_have_steps_left(ask):
+    """Equal exponents: every launch but the last holds `resident` slots."""
+    for slots, resident, steps, chunk in ((37, 18, 30, 1), (150, 148, 24, 3), (7, 3, 10, 4)):
+        lines = ask(f"split {slots} {resident} {steps} {chunk} " + " ".join(["0"] * slots + [str(steps)] * slots))[:-1]
+        rounds = -(-steps // chunk)
+        assert len(lines) == -(-slots * rounds // resident)
+        assert all(len(line.split(":")[1].split()) == resident for line in lines[:-1])
