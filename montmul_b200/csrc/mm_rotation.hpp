@@ -18,14 +18,16 @@ namespace mm {
 // work of one); in rotation the idle places go to the next round's slots and only the last launch
 // is partly empty. A launch costs launch_us beyond its steps (its start, and the wait for its slowest
 // block), so a chunk is no shorter than pays for that: 13 us measured for clusters (one block per
-// SM), about 90 us in shared memory, where an SM's blocks finish at different times.
+// SM), about 90 us in shared memory, where an SM's blocks finish at different times. The chunks
+// tried are those of 64 numbers of rounds, from the fewest that `most` steps per launch allow: past
+// that the last launch's idle places no longer count.
 inline size_t rotation_chunk(size_t slots, size_t resident, size_t steps, size_t most, double step_us, double launch_us) {
     if (slots <= resident || slots % resident == 0 || slots > 16 * resident) return 0;
     double best = 0.97 * (double)((slots + resident - 1) / resident) * (double)steps * step_us;
     size_t chunk = 0;
-    for (size_t r = 1; r <= 64 && r <= steps; ++r) {
+    const size_t fewest = (steps + most - 1) / most;
+    for (size_t r = fewest; r < fewest + 64 && r <= steps; ++r) {
         const size_t s = (steps + r - 1) / r, rounds = (steps + s - 1) / s;
-        if (s > most) continue;
         const size_t launches = (slots * rounds + resident - 1) / resident;
         const double us = (double)launches * ((double)s * step_us + launch_us);
         if (us < best) {

@@ -96,3 +96,19 @@ def test_queued_runs_in_rotation_do_not_wait_on_the_host(gpu):
     assert be.launches(st) - before > 4
     be.sync(st)
     assert host < 0.5 * one, (host, one)
+
+
+def test_rotation_in_a_run_of_many_launches(gpu):
+    """More than 64 launches' worth of steps: still in rotation (71 launches of 148 slots; one launch over
+    all slots after another would be 70)."""
+    slots, steps = 150, 140
+    nbits = [steps - i % 3 for i in range(slots)]
+    a, b = batch(gpu, 200_000, slots, nbits), batch(gpu, 200_000, slots, nbits)
+    be, st = a.backend_and_state()
+    be.set_schedule(st, 0, 2)
+    before = be.launches(st)
+    a.run(steps)
+    assert gpu.sm_count() != 148 or be.launches(st) - before == 71
+    for _ in range(steps):
+        b.run(1)
+    assert np.array_equal(raw(a), raw(b))

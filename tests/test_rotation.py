@@ -96,3 +96,14 @@ def test_full_launches_while_enough_slots_have_steps_left(ask):
         rounds = -(-steps // chunk)
         assert len(lines) == -(-slots * rounds // resident)
         assert all(len(line.split(":")[1].split()) == resident for line in lines[:-1])
+
+
+# (slots, resident, steps per launch at most, us per step): 2,368 slots at L = 1,024, 500 at L = 8,192,
+# 37 clusters of L = 65,536, 150 slots at L = 16,384.
+@pytest.mark.parametrize("slots,resident,most,us", [(2368, 888, 64, 94.0), (500, 296, 64, 186.0), (37, 36, 512, 370.0), (150, 148, 512, 223.0)])
+def test_rotation_does_not_depend_on_the_length_of_a_run(ask, slots, resident, most, us):
+    for steps in (200, 65 * most, 100_000, 1_000_000):
+        chunk = int(ask(f"chunk {slots} {resident} {steps} {most} {us} 20")[0])
+        assert 0 < chunk <= min(most, steps)
+        launches = -(-slots * -(-steps // chunk) // resident)
+        assert launches * (chunk * us + 20) < 1.05 * slots / resident * steps * us + chunk * us
