@@ -376,8 +376,10 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         most = std::max(most, (size_t)(b->nbits[i] - b->pos[i]));
         active += b->pos[i] < b->nbits[i];
     }
-    size_t left = std::min(bits, most);
+    const size_t left = std::min(bits, most);
     if (left == 0) return MM_OK;
+    size_t work = 0;
+    for (size_t i = 0; i < b->slots; ++i) work += std::min(left, (size_t)(b->nbits[i] - b->pos[i]));
     int rc = push(b);
     if (rc) return rc;
     SlotArgs a = slot_args(b);
@@ -424,7 +426,13 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     // A step of one launch's resident slots: the schedule's time per slot-step at full occupancy
     // times their number, else a model of the transform work.
     const double step_us = b->sched.step_ns > 0 ? 1e-3 * b->sched.step_ns * (double)resident : 1e-3 * (double)b->n * b->m;
-    const size_t turn = rotation_chunk(active, resident, left, chunk, step_us, b->global ? 13.0 : 90.0);
+    const double launch_us = b->global ? 13.0 : 90.0;
+    size_t turn = rotation_chunk(active, resident, left, chunk, step_us, launch_us);
+    if (turn && 8 * work < 7 * b->slots * left) {   // exponents of different lengths
+        std::vector<uint32_t> rem(b->slots);
+        for (size_t i = 0; i < b->slots; ++i) rem[i] = (uint32_t)std::min(left, (size_t)(b->nbits[i] - b->pos[i]));
+        if (!rotation_pays(rem, resident, left, chunk, turn, step_us, launch_us)) turn = 0;
+    }
     // Without a rotation each launch takes every slot once.
     Rotation rot(b->slots, turn ? resident : b->slots, left, turn ? turn : std::min(left, chunk));
     StepRange r;

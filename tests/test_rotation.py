@@ -1,6 +1,7 @@
 """How run splits its steps into launches (montmul_b200/csrc/mm_rotation.hpp, built for the host with
 g++): every slot gets the steps it has left, no more than the device holds are stepped at once, and
 no slot is in a launch twice, for any slot counts and exponents. CPU only."""
+import heapq
 import os
 import random
 import shutil
@@ -15,6 +16,7 @@ SOURCE = r'''
 #include <cstring>
 #include <vector>
 // "split slots resident steps chunk pos... nbits...": one line per launch, "first bits bits_next: slot/steps ...".
+// "pays slots resident steps most chunk step_us launch_us left...": 1 or 0.
 // "chunk slots resident steps most step_us launch_us": the rotation's steps per launch.
 int main() {
     char what[16];
@@ -24,6 +26,15 @@ int main() {
             double step_us, launch_us;
             if (std::scanf("%lf %lf", &step_us, &launch_us) != 2) return 1;
             std::printf("%zu\n", mm::rotation_chunk(slots, resident, steps, last, step_us, launch_us));
+            continue;
+        }
+        if (!std::strcmp(what, "pays")) {
+            size_t chunk;
+            double step_us, launch_us;
+            if (std::scanf("%zu %lf %lf", &chunk, &step_us, &launch_us) != 3) return 1;
+            std::vector<uint32_t> left(slots);
+            for (auto& v : left) if (std::scanf("%u", &v) != 1) return 1;
+            std::printf("%d\n", (int)mm::rotation_pays(left, resident, steps, last, chunk, step_us, launch_us));
             continue;
         }
         std::vector<uint32_t> pos(slots), nbits(slots);
@@ -107,3 +118,57 @@ def test_rotation_does_not_depend_on_the_length_of_a_run(ask, slots, resident, m
         assert 0 < chunk <= min(most, steps)
         launches = -(-slots * -(-steps // chunk) // resident)
         assert launches * (chunk * us + 20) < 1.05 * slots / resident * steps * us + chunk * us
+
+
+def whole_time(left, resident, most, us, launch_us):
+    """One launch over all slots after another: blocks start in order as places come free."""
+    t, left = 0.0, list(left)
+    while any(left):
+        ends = [0.0] * resident
+        for r in left:
+            if r:
+                heapq.heapreplace(ends, ends[0] + min(r, most) * us)
+        t += max(ends) + launch_us
+        left = [r - min(r, most) for r in left]
+    return t
+
+
+def rotation_time(ask, left, resident, steps, chunk, us, launch_us):
+    """Launch after launch, each as long as its longest slot."""
+    t, left = 0.0, list(left)
+    for line in ask(f"split {len(left)} {resident} {steps} {chunk} " + " ".join(["0"] * len(left) + list(map(str, left))))[:-1]:
+        longest = 0
+        for w in line.split(":")[1].split():
+            s, b = map(int, w.split("/"))
+            longest = max(longest, min(b, left[s]))
+            left[s] -= min(b, left[s])
+        t += longest * us + launch_us
+    return t
+
+
+def test_rotation_of_unequal_exponents_pays_where_it_is_taken(ask):
+    """Random exponent lengths: where rotation_pays takes a rotation it is not slower than launches over
+    all slots (by both models written out), and it does take some."""
+    rng = random.Random(7)
+    taken = slower = 0
+    for _ in range(150):
+        resident = rng.choice([18, 36, 148])
+        slots = int(resident * rng.uniform(1.02, 4))
+        steps, most, us = rng.choice([100, 300, 1000]), rng.choice([64, 512]), rng.choice([20, 100, 400])
+        share, lo = rng.random(), rng.randint(0, steps)
+        kind = rng.choice(["two", "even", "sorted"])
+        left = [steps if rng.random() < share else (lo if kind != "even" else rng.randint(0, steps)) for _ in range(slots)]
+        left[rng.randrange(slots)] = steps
+        if kind == "sorted":
+            left.sort()
+        active = sum(v > 0 for v in left)
+        chunk = int(ask(f"chunk {active} {resident} {steps} {most} {us} 20")[0])
+        if not chunk:
+            continue
+        ratio = rotation_time(ask, left, resident, steps, chunk, us, 20) / whole_time(left, resident, most, us, 0)
+        if ask(f"pays {slots} {resident} {steps} {most} {chunk} {us} 20 " + " ".join(map(str, left)))[0] == "1":
+            taken += 1
+            assert ratio < 1.02, (ratio, slots, resident, steps, most, us, left)
+        else:
+            slower += ratio > 1.05
+    assert taken > 20 and slower > 5
