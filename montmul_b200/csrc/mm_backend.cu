@@ -427,7 +427,8 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     // times their number, else a model of the transform work.
     const double step_us = b->sched.step_ns > 0 ? 1e-3 * b->sched.step_ns * (double)resident : 1e-3 * (double)b->n * b->m;
     const double launch_us = b->global ? 13.0 : 90.0;
-    size_t turn = rotation_chunk(active, resident, left, chunk, step_us, launch_us);
+    const double half_wave = !b->global && step_fn == b->ks.step && b->m == 12 ? 0.53 : 1.0;
+    size_t turn = rotation_chunk(active, resident, left, chunk, step_us, launch_us, half_wave);
     if (turn && 8 * work < 7 * b->slots * left) {   // exponents of different lengths
         std::vector<uint32_t> rem(b->slots);
         for (size_t i = 0; i < b->slots; ++i) rem[i] = (uint32_t)std::min(left, (size_t)(b->nbits[i] - b->pos[i]));

@@ -24,9 +24,15 @@ namespace mm {
 // SM), about 90 us in shared memory, where an SM's blocks finish at different times. The chunks
 // tried are those of 64 numbers of rounds, from the fewest that `most` steps per launch allow: past
 // that the last launch's idle places no longer count.
-inline size_t rotation_chunk(size_t slots, size_t resident, size_t steps, size_t most, double step_us, double launch_us) {
+// half_wave: a step of a launch that fills at most half the places, of a full one's. 1 where a step is as
+// long however few blocks an SM holds; at L = 8192, two blocks per SM of which one alone keeps the
+// pipes nearly as busy, 0.53 (97 us against 2 x 91). There a last wave that is half full idles little:
+// in rotation 444 slots took 1.005 and 1,006 slots (3.4 waves) 1.008 to 1.04 times as long.
+inline size_t rotation_chunk(size_t slots, size_t resident, size_t steps, size_t most, double step_us, double launch_us,
+                             double half_wave) {
     if (slots <= resident || slots % resident == 0 || slots > 16 * resident) return 0;
-    double best = 0.97 * (double)((slots + resident - 1) / resident) * (double)steps * step_us;
+    const size_t full = slots / resident, rest = slots % resident;
+    double best = 0.97 * ((double)full + (2 * rest <= resident ? half_wave : 1.0)) * (double)steps * step_us;
     size_t chunk = 0;
     const size_t fewest = (steps + most - 1) / most;
     for (size_t r = fewest; r < fewest + 64 && r <= steps; ++r) {

@@ -17,15 +17,15 @@ SOURCE = r'''
 #include <vector>
 // "split slots resident steps chunk pos... nbits...": one line per launch, "first bits bits_next: slot/steps ...".
 // "pays slots resident steps most chunk step_us launch_us left...": 1 or 0.
-// "chunk slots resident steps most step_us launch_us": the rotation's steps per launch.
+// "chunk slots resident steps most step_us launch_us half_wave": the rotation's steps per launch.
 int main() {
     char what[16];
     size_t slots, resident, steps, last;
     while (std::scanf("%15s %zu %zu %zu %zu", what, &slots, &resident, &steps, &last) == 5) {
         if (!std::strcmp(what, "chunk")) {
-            double step_us, launch_us;
-            if (std::scanf("%lf %lf", &step_us, &launch_us) != 2) return 1;
-            std::printf("%zu\n", mm::rotation_chunk(slots, resident, steps, last, step_us, launch_us));
+            double step_us, launch_us, half_wave;
+            if (std::scanf("%lf %lf %lf", &step_us, &launch_us, &half_wave) != 3) return 1;
+            std::printf("%zu\n", mm::rotation_chunk(slots, resident, steps, last, step_us, launch_us, half_wave));
             continue;
         }
         if (!std::strcmp(what, "pays")) {
@@ -114,7 +114,7 @@ def test_full_launches_while_enough_slots_have_steps_left(ask):
 @pytest.mark.parametrize("slots,resident,most,us", [(2368, 888, 64, 94.0), (500, 296, 64, 186.0), (37, 36, 512, 370.0), (150, 148, 512, 223.0)])
 def test_rotation_does_not_depend_on_the_length_of_a_run(ask, slots, resident, most, us):
     for steps in (200, 65 * most, 100_000, 1_000_000):
-        chunk = int(ask(f"chunk {slots} {resident} {steps} {most} {us} 20")[0])
+        chunk = int(ask(f"chunk {slots} {resident} {steps} {most} {us} 20 1")[0])
         assert 0 < chunk <= min(most, steps)
         launches = -(-slots * -(-steps // chunk) // resident)
         assert launches * (chunk * us + 20) < 1.05 * slots / resident * steps * us + chunk * us
@@ -162,7 +162,7 @@ def test_rotation_of_unequal_exponents_pays_where_it_is_taken(ask):
         if kind == "sorted":
             left.sort()
         active = sum(v > 0 for v in left)
-        chunk = int(ask(f"chunk {active} {resident} {steps} {most} {us} 20")[0])
+        chunk = int(ask(f"chunk {active} {resident} {steps} {most} {us} 20 1")[0])
         if not chunk:
             continue
         ratio = rotation_time(ask, left, resident, steps, chunk, us, 20) / whole_time(left, resident, most, us, 0)
@@ -172,3 +172,12 @@ def test_rotation_of_unequal_exponents_pays_where_it_is_taken(ask):
         else:
             slower += ratio > 1.05
     assert taken > 20 and slower > 5
+
+
+def test_half_full_last_wave_at_8192(ask):
+    """Two blocks per SM, one alone at 0.94 of their rate: waves of 0.1 and 0.8 of the places are taken in
+    rotation, a last wave near half full is not."""
+    chunk = lambda slots, half: int(ask(f"chunk {slots} 296 256 64 186 90 {half}")[0])
+    for slots, rotates in ((301, True), (370, True), (444, False), (540, True), (800, True), (1006, False)):
+        assert (chunk(slots, 0.53) > 0) == rotates, slots
+    assert all(chunk(slots, 1) > 0 for slots in (301, 370, 444, 540, 800, 1006))
