@@ -188,7 +188,8 @@ void mm_b200_t_free(mm_b200_tbuf *b);
  * the launches of run when a batch has so few slots that SMs would idle; L = 4096,
  * 8192 and 16384 also build one alternative shape); in cluster mode, threads per SM (0 or 512:
  * one 512-thread block of 8192 elements per SM; 1024 at L = 32768: two 512-thread blocks of 4096
- * elements per SM, a cluster of 4). get_schedule reports the shape in use. The autotuner
+ * elements per SM, a cluster of 4). get_schedule reports the schedule: its mode and its block shape,
+ * which item lists and plans run; last_run reports what run's launches took. The autotuner
  * (montmul_b200.tune) measures these per length and caches them. */
 typedef struct {
     int global;
@@ -198,6 +199,17 @@ typedef struct {
 } mm_b200_schedule;
 int mm_b200_set_schedule(mm_b200_batch *b, const mm_b200_schedule *s);
 int mm_b200_get_schedule(const mm_b200_batch *b, mm_b200_schedule *s);
+/* What the launches of the batch's last run, run_async or run_bare with steps to do took: mode (as
+ * in the schedule), threads per block, blocks per slot (cluster mode; else 1), and the most slots
+ * with steps left that one launch steps: all slots, or fewer when run takes them in rotation. All 0
+ * before the first run. */
+typedef struct {
+    int mode;
+    int threads;
+    int blocks;
+    size_t slots;
+} mm_b200_run_info;
+int mm_b200_last_run(const mm_b200_batch *b, mm_b200_run_info *info);
 
 /* ---- In-place refill (no counterpart in the reference): a serving loop replaces finished
  * slots while the others keep their state on the device. ----

@@ -69,6 +69,7 @@ SIGNATURES = {
     "mm_b200_bfly_peak": ([C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)], C.c_int),
     "mm_b200_set_schedule": ([_vp, _vp], C.c_int),
     "mm_b200_get_schedule": ([_vp, _vp], C.c_int),
+    "mm_b200_last_run": ([_vp, _vp], C.c_int),
     "mm_b200_set_moduli": ([_vp, _sz, _vp, _vp, _vp], C.c_int),
     "mm_b200_write_slots": ([_vp, _sz, _vp, _vp, _vp, _sz, _vp], C.c_int),
     "mm_b200_read_slots": ([_vp, _sz, _vp, _vp], C.c_int),
@@ -121,6 +122,11 @@ class TBuf:
 class Schedule(C.Structure):
     """mm_b200_schedule: global mode, steps per launch, measured ns per slot-step."""
     _fields_ = [("global_", C.c_int), ("launch_steps", C.c_int), ("step_ns", C.c_double), ("threads", C.c_int)]
+
+
+class RunInfo(C.Structure):
+    """mm_b200_run_info: what the launches of a batch's last run took."""
+    _fields_ = [("mode", C.c_int), ("threads", C.c_int), ("blocks", C.c_int), ("slots", _sz)]
 
 
 def _ptr(a):
@@ -374,6 +380,13 @@ class B200:
         _check(lib().mm_b200_get_schedule(st.ptr, C.byref(sc)))
         return {"global": bool(sc.global_), "mode": ("shared", "global", "cluster")[sc.global_],
                 "launch_steps": sc.launch_steps, "step_ns": sc.step_ns, "threads": sc.threads}
+
+    def last_run(self, st):
+        """What the last run's launches took: mode, threads per block, blocks per slot, and the
+        slots one launch steps (fewer than the batch has in a rotation)."""
+        r = RunInfo()
+        _check(lib().mm_b200_last_run(st.ptr, C.byref(r)))
+        return {"mode": ("shared", "global", "cluster")[r.mode], "threads": r.threads, "blocks": r.blocks, "slots": r.slots}
 
     def set_moduli(self, st, slots, n, nprime):
         ids = np.ascontiguousarray(slots, np.uintp)

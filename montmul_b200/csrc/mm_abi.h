@@ -79,6 +79,7 @@ GlobalKernels global_kernels();       // mm_global.cu
 // memory opt-in on the current device; cluster_launch runs `bits` steps on every slot of a batch.
 constexpr int kMinClusterLogN = 14;
 constexpr int kMaxClusterLogN = 15;
+constexpr int kClusterThreads = 512;        // threads per block
 constexpr int kClusterChunkLog = 13;        // the default chunk
 constexpr int kClusterPairChunkLog = 12;    // the two-blocks-per-SM chunk, at L = 32768
 // kClusterWideLogN (L = 131072, eight blocks): not a mode a schedule names; run takes it for

@@ -132,6 +132,7 @@ struct mm_b200_batch {
     std::vector<uint32_t> nbits, pos;
     bool exp_dirty = false;
     uint64_t launches = 0;
+    mm_b200_run_info last_run{0, 0, 0, 0};
     uint2* d_items = nullptr;          // run_items: the list on the device and its pinned staging
     uint2* h_items = nullptr;
     cudaEvent_t items_copied = nullptr;   // the staging may be rewritten once this has passed
@@ -436,6 +437,10 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     }
     // Without a rotation each launch takes every slot once.
     Rotation rot(b->slots, turn ? resident : b->slots, left, turn ? turn : std::min(left, chunk));
+    if (clustered) b->last_run = {2, kClusterThreads, 1 << (b->m - b->cluster_chunk_log), 0};
+    else if (b->global) b->last_run = {1, b->gk.threads, 1, 0};
+    else b->last_run = {0, step_threads, 1, 0};
+    b->last_run.slots = turn ? resident : b->slots;
     StepRange r;
     size_t count = 0;
     while (rot.next(b->pos.data(), b->nbits.data(), &r, &count)) {
@@ -1027,6 +1032,12 @@ int mm_b200_set_schedule(mm_b200_batch* b, const mm_b200_schedule* sc) {
 int mm_b200_get_schedule(const mm_b200_batch* b, mm_b200_schedule* sc) {
     if (!b || !sc) return fail(MM_ERR_ARG, "get_schedule: null argument");
     *sc = b->sched;
+    return MM_OK;
+}
+
+int mm_b200_last_run(const mm_b200_batch* b, mm_b200_run_info* info) {
+    if (!b || !info) return fail(MM_ERR_ARG, "last_run: null argument");
+    *info = b->last_run;
     return MM_OK;
 }
 

@@ -25,7 +25,6 @@ namespace cgx = cooperative_groups;
 
 constexpr int kChunkLog = kClusterChunkLog;     // elements per CTA by default: 2^13
 constexpr int kChunk = 1 << kChunkLog;
-constexpr int kClusterThreads = 512;
 constexpr int kClusterSmem = 24 * kChunk;      // 192 KiB
 
 // The chunks of every CTA of the cluster, as generic pointers (the own chunk included).

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import common
-from montmul_b200 import ModBatch
+from montmul_b200 import ModBatch, tune
 
 pytestmark = pytest.mark.gpu
 
@@ -34,8 +34,20 @@ def raw(b):
     return np.array(be.read_all(st))
 
 
-# Transform lengths with wide shapes (L = 128 to 4096): the top of a bucket, an odd size, and
-# more slots than the widest shape holds at once (which takes the next one).
+def ran(b):
+    """What the launches of the batch's last run took."""
+    be, st = b.backend_and_state()
+    return be.last_run(st)
+
+
+def wide_threads(length):
+    """Threads of the default shape and of the wide ones, widest first (mm_abi.h wide_threads_for)."""
+    default = tune.threads_for(length.bit_length() - 2)
+    return default, [f * default for f in (4, 2) if f * default <= 512]
+
+
+# Transform lengths with wide shapes (L = 128 to 4096): the top of a bucket and odd sizes. test_each_wide_shape
+# has the slot counts at which each shape runs.
 @pytest.mark.parametrize("bits,slots", [(16 * (1 << e) - 4, s) for e in range(7, 13) for s in (1, 3)] +
                          [(1500, 2), (4097, 400), (9001, 300), (33_000, 160)])
 def test_wide_shapes_same_raw_as_default_shape(gpu, bits, slots):
@@ -45,7 +57,56 @@ def test_wide_shapes_same_raw_as_default_shape(gpu, bits, slots):
     be.set_schedule(st, 0, 0, 0.0, be.get_schedule(st)["threads"])   # a named shape stays
     a.run(100)
     b.run(100)
+    default, wide = wide_threads(a.params.len)
+    assert ran(b)["threads"] == default
+    if slots <= gpu.sm_count():
+        assert ran(a)["threads"] == wide[0]
     assert np.array_equal(raw(a), raw(b))
+
+
+@pytest.mark.parametrize("length", [1 << e for e in range(7, 13)])
+def test_each_wide_shape(gpu, length):
+    """The slot counts of each shape: the widest one up to a block of 512 threads (or blocks of that many
+    together) per SM, the next one beyond, the default from five per SM on."""
+    sms = gpu.sm_count()
+    default, wide = wide_threads(length)
+    seen = []
+    for slots in (sms * (512 // wide[0]), sms * (512 // wide[0]) + 1, 5 * sms + 1):
+        nbits = [9 + i % 3 for i in range(slots)]
+        a, b = batch(gpu, 16 * length - 4, slots, nbits), batch(gpu, 16 * length - 4, slots, nbits)
+        be, st = b.backend_and_state()
+        be.set_schedule(st, 0, 0, 0.0, default)
+        a.run(100)
+        b.run(100)
+        seen.append(ran(a)["threads"])
+        assert ran(b)["threads"] == default and np.array_equal(raw(a), raw(b))
+    assert seen == [wide[0], (wide + [default])[1], default]
+
+
+class Pinned:
+    """A device whose batches name the default block shape of their length."""
+
+    def __init__(self, dev):
+        self.dev = dev
+
+    def __getattr__(self, name):
+        return getattr(self.dev, name)
+
+    def create(self, *a):
+        st = self.dev.create(*a)
+        self.dev.set_schedule(st, 0, 0, 0.0, self.dev.get_schedule(st)["threads"])
+        return st
+
+
+@pytest.mark.parametrize("wraparound", [True, False])
+@pytest.mark.parametrize("length", [1 << e for e in range(7, 13)])
+def test_default_shape_same_raw_as_oracle(oracle, length, wraparound):
+    """The shape that full batches run, on few slots: at the top of the bucket and just above the one below."""
+    from montmul_b200 import B200
+    make = oracle.OracleBackend.wraparound if wraparound else oracle.OracleBackend.plain
+    dev = Pinned(B200(wraparound=wraparound))
+    common.same_raw(lambda: dev, make, 16 * length - 36, 2, 12)
+    common.same_raw(lambda: dev, make, 8 * length + 1, 3, 12)
 
 
 # L = 16384 holds one slot per SM, L = 32768 and 65536 a cluster per 2 and 4 SMs: a few slots
@@ -59,6 +120,7 @@ def test_rotation_same_raw_as_single_steps(gpu, bits, slots, steps):
     before = be.launches(st)
     a.run(steps)
     assert be.launches(st) - before > 1 and all(a.remaining(i) == 0 for i in range(slots))
+    assert ran(a)["slots"] < slots
     for _ in range(steps):
         b.run(1)
     assert np.array_equal(raw(a), raw(b))
@@ -74,6 +136,7 @@ def test_clusters_of_eight_same_raw_as_global_mode(gpu):
         plan.run(6)
         plan.close()
         assert a.params.len == 131072 and np.array_equal(raw(a), raw(b))
+        assert (ran(a)["mode"], ran(a)["blocks"]) == ("cluster", 8)
 
 
 def test_queued_runs_in_rotation_do_not_wait_on_the_host(gpu):
@@ -112,3 +175,30 @@ def test_rotation_in_a_run_of_many_launches(gpu):
     for _ in range(steps):
         b.run(1)
     assert np.array_equal(raw(a), raw(b))
+
+
+# (bits, wraparound, forced global, slots per SM, more slots, steps): several blocks per SM, the plain REDC,
+# the global-mode kernel, clusters of eight (18 of them on 148 SMs).
+@pytest.mark.parametrize("bits,wrap,forced,per_sm,more,steps", [
+    (8_000, True, False, 16, 40, 40), (12_000, True, False, 6, 10, 40), (20_011, False, False, 2, 5, 40), (131_068, True, True, 2, 1, 12),
+    (2_097_148, True, False, 0, 25, 4)])
+def test_rotation_in_every_mode(bits, wrap, forced, per_sm, more, steps):
+    from montmul_b200 import B200
+    dev = B200(wraparound=wrap, force_global=forced)
+    slots = per_sm * dev.sm_count() + more
+    nbits = [steps if i % 9 else 1 + i % steps for i in range(slots)]
+    a, b = batch(dev, bits, slots, nbits, base=2), batch(dev, bits, slots, nbits, base=2)
+    a.run(steps)
+    assert ran(a)["slots"] < slots
+    for _ in range(steps):
+        b.run(1)
+    assert np.array_equal(raw(a), raw(b))
+
+
+def test_bare_steps_in_rotation_leave_x_alone(gpu):
+    slots, steps = 150, 24
+    b = batch(gpu, 200_000, slots, [steps] * slots)
+    before = raw(b)
+    be, st = b.backend_and_state()
+    be.run_bare(st, steps)
+    assert ran(b)["slots"] < slots and np.array_equal(raw(b), before) and b.remaining(0) == 0
