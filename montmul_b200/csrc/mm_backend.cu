@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -83,6 +84,7 @@ struct mm_b200_device {
     std::map<int, bool> configured;
     std::map<const void*, int> resident;   // blocks of a step kernel that the device holds at once
     std::map<int, int> resident_clusters;  // the same of cluster mode, by 32 m + chunk_log
+    std::vector<mm_b200_batch*> batches;   // every batch of the device
 };
 
 struct mm_b200_batch {
@@ -110,6 +112,8 @@ struct mm_b200_batch {
     cudaEvent_t stage_copied = nullptr;   // the last host-to-device copy out of h_stage
     size_t hstage_cap = 0;
     cudaStream_t stream = nullptr;
+    cudaEvent_t paced = nullptr;          // the end of the last launch of a run in a wide shape
+    std::atomic<bool> stepping{false};    // steps were enqueued and not waited for since
     uint32_t* d_x = nullptr;
     uint32_t* d_t = nullptr;
     F2* d_c2 = nullptr;
@@ -272,6 +276,7 @@ int check_err(mm_b200_batch* b, const char* what) {
     std::vector<uint32_t> err(b->slots);
     MM_CK(cudaMemcpyAsync(err.data(), b->d_err, b->slots * 4, cudaMemcpyDeviceToHost, b->stream));
     MM_CK(cudaStreamSynchronize(b->stream));
+    b->stepping = false;
     for (size_t i = 0; i < b->slots; ++i) {
         if (err[i]) {
             MM_CK(cudaMemsetAsync(b->d_err, 0, b->slots * 4, b->stream));
@@ -324,26 +329,45 @@ int resident_blocks(mm_b200_batch* b, StepFn fn, int threads, int* out) {
     return MM_OK;
 }
 
-// The block shape of run's launches over `active` slots in shared memory: the widest one whose
-// blocks are all resident at once, at most five per SM, unless the schedule fixes the shape. With
+// Slots of the device's other batches that may be stepping beside b's: of those with steps under way (runs, item
+// lists, plans), or with `alive` of all. As good as infinitely many if one is not of b's length in
+// shared memory.
+size_t slots_beside(mm_b200_batch* b, bool alive) {
+    // Another thread's stream capture does not concern these streams.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    size_t beside = 0;
+    {
+        std::lock_guard<std::mutex> lock(b->dev->mu);
+        for (mm_b200_batch* o : b->dev->batches) {
+            if (o == b || !(alive || (o->stepping && cudaStreamQuery(o->stream) == cudaErrorNotReady))) continue;
+            beside += o->m == b->m && !o->global ? o->slots : ~(size_t)0 / 2 / b->dev->batches.size();
+        }
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return beside;
+}
+
+// The wide block shape for `active` slots in shared memory: the widest one whose blocks are all
+// resident at once, at most five per SM; none where the schedule fixes the shape. With
 // every slot resident the time of a run is one slot's, which more threads shorten (ms for 500 steps
 // at L = 512, default 32 threads -> wide: 64 slots 22.5 -> 14.5, 592 slots 23.4 -> 16.8; 300 steps at L = 1024,
 // 592 slots: 18.2 -> 13.7; 200 steps at L = 4096, 148 slots: 13.8 -> 10.7). With more slots the default
 // shape's rate per SM is higher (L = 512, 64 threads: 700 slots 24 -> 18.1, 1,000 slots 24.2 -> 26.8).
-// Item lists (run_items) keep the default shape: a serving loop runs several of them at the same
-// time, which fill the SMs together.
-int step_shape(mm_b200_batch* b, size_t active, StepFn* fn, int* threads) {
-    *fn = b->step_fn;
-    *threads = b->step_threads;
-    if (b->step_fixed) return MM_OK;
+// Slots of other batches that run at the same time count like the batch's own (slots_beside; four batches of 148
+// slots at L = 1024, 300 steps each under run_async: 24.8 ms in the default shape, 36.6 in wide ones).
+// Item lists (run_items) always take the default shape: a serving loop runs several of them at the
+// same time.
+int wide_shape(mm_b200_batch* b, size_t active, const WideShape** out) {
+    *out = nullptr;
+    if (b->step_fixed || b->global) return MM_OK;
     for (const WideShape& w : b->ks.wide) {
         if (!w.step) continue;
         int res = 0;
         const int rc = resident_blocks(b, w.step, w.threads, &res);
         if (rc) return rc;
         if (active <= (size_t)std::min(res, 5 * b->dev->sms)) {
-            *fn = w.step;
-            *threads = w.threads;
+            *out = &w;
             return MM_OK;
         }
     }
@@ -371,7 +395,13 @@ int resident_slots(mm_b200_batch* b, bool clustered, StepFn fn, int threads, siz
     return MM_OK;
 }
 
-int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
+// Steps per launch of a run in a wide shape that waits for its launches.
+constexpr size_t kPacedSteps = 128;
+
+// Enqueues up to `bits` steps on every slot. `waits`: the caller waits for them. A run that may take a wide
+// shape then enqueues each launch after the one before, in the shape that suits what else is under
+// way by then; without, it takes all other batches of the device to run beside it.
+int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
     size_t most = 0, active = 0;
     for (size_t i = 0; i < b->slots; ++i) {
         most = std::max(most, (size_t)(b->nbits[i] - b->pos[i]));
@@ -400,12 +430,13 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         c.tab2 = b->ctab->t2;
         c.tab1 = b->ctab->t1;
     }
-    StepFn step_fn = nullptr;
-    int step_threads = 0;
-    if (!b->global) {
-        rc = step_shape(b, active, &step_fn, &step_threads);
-        if (rc) return rc;
-    }
+    const WideShape* wide = nullptr;
+    rc = wide_shape(b, active + (waits ? 0 : slots_beside(b, true)), &wide);
+    if (rc) return rc;
+    const bool paced = wide && waits;
+    if (paced && !b->paced) MM_CK(cudaEventCreateWithFlags(&b->paced, cudaEventDisableTiming));
+    StepFn step_fn = wide ? wide->step : b->step_fn;
+    int step_threads = wide ? wide->threads : b->step_threads;
     // One launch over the first `count` slots of a range.
     const auto launch = [&](size_t count, const StepRange& r) -> int {
         if (clustered) {
@@ -420,8 +451,10 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
         ++b->launches;
         return MM_OK;
     };
-    const size_t chunk = (size_t)std::max(1, b->sched.launch_steps > 0 ? b->sched.launch_steps : b->dev->max_launch_steps);
+    size_t chunk = (size_t)std::max(1, b->sched.launch_steps > 0 ? b->sched.launch_steps : b->dev->max_launch_steps);
+    if (paced) chunk = std::min(chunk, kPacedSteps);
     size_t resident = 0;
+    b->stepping = true;
     rc = resident_slots(b, clustered, step_fn, step_threads, &resident);
     if (rc) return rc;
     // A step of one launch's resident slots: the schedule's time per slot-step at full occupancy
@@ -443,9 +476,18 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare = false) {
     b->last_run.slots = turn ? resident : b->slots;
     StepRange r;
     size_t count = 0;
-    while (rot.next(b->pos.data(), b->nbits.data(), &r, &count)) {
+    for (bool first = true; rot.next(b->pos.data(), b->nbits.data(), &r, &count); first = false) {
+        if (paced) {
+            if (!first) MM_CK(cudaEventSynchronize(b->paced));
+            rc = wide_shape(b, active + slots_beside(b, false), &wide);
+            if (rc) return rc;
+            step_fn = wide ? wide->step : b->step_fn;
+            step_threads = wide ? wide->threads : b->step_threads;
+            b->last_run.threads = step_threads;
+        }
         rc = launch(count, r);
         if (rc) return rc;
+        if (paced) MM_CK(cudaEventRecord(b->paced, b->stream));
         rot.advance(r, count, b->pos.data(), b->nbits.data());
     }
     if (!bare) b->host_x_valid = false;
@@ -688,6 +730,10 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     // On a failure below, everything allocated so far is released with the batch.
     std::unique_ptr<mm_b200_batch, void (*)(mm_b200_batch*)> b(new mm_b200_batch(), mm_b200_destroy);
     b->dev = dev;
+    {
+        std::lock_guard<std::mutex> lock(dev->mu);
+        dev->batches.push_back(b.get());
+    }
     b->m = m;
     b->k = k;
     b->n = len / 2;
@@ -811,7 +857,7 @@ int mm_b200_set_exponents(mm_b200_batch* b, const uint32_t* words, size_t ew, co
 int mm_b200_run_async(mm_b200_batch* b, size_t bits) {
     if (!b) return fail(MM_ERR_ARG, "run: null batch");
     MM_CK(cudaSetDevice(b->dev->device));
-    return launch_steps(b, bits);
+    return launch_steps(b, bits, false, false);
 }
 
 int mm_b200_push(mm_b200_batch* b) {
@@ -829,13 +875,15 @@ int mm_b200_sync(mm_b200_batch* b) {
 int mm_b200_run_bare(mm_b200_batch* b, size_t bits) {
     if (!b) return fail(MM_ERR_ARG, "run_bare: null batch");
     MM_CK(cudaSetDevice(b->dev->device));
-    int rc = launch_steps(b, bits, true);
+    int rc = launch_steps(b, bits, true, true);
     if (rc) return rc;
     return mm_b200_sync(b);
 }
 
 int mm_b200_run(mm_b200_batch* b, size_t bits) {
-    int rc = mm_b200_run_async(b, bits);
+    if (!b) return fail(MM_ERR_ARG, "run: null batch");
+    MM_CK(cudaSetDevice(b->dev->device));
+    int rc = launch_steps(b, bits, false, true);
     if (rc) return rc;
     return mm_b200_sync(b);
 }
@@ -883,6 +931,7 @@ int mm_b200_run_items_async(mm_b200_batch* b, size_t count, const size_t* slots,
     MM_CK(cudaMemcpyAsync(b->d_items, b->h_items, count * sizeof(uint2), cudaMemcpyHostToDevice, b->stream));
     MM_CK(cudaEventRecord(b->items_copied, b->stream));
     SlotArgs a = slot_args(b);
+    b->stepping = true;
     for (size_t first = 0; first < count; first += 65535) {
         const unsigned grid = (unsigned)std::min<size_t>(65535, count - first);
         b->step_fn<<<grid, b->step_threads, b->ks.smem, b->stream>>>(a, StepRange{}, b->d_items + first);
@@ -951,6 +1000,11 @@ uint64_t mm_b200_launches(const mm_b200_batch* b) { return b ? b->launches : 0; 
 void mm_b200_destroy(mm_b200_batch* b) {
     if (!b) return;
     cudaSetDevice(b->dev->device);
+    {
+        std::lock_guard<std::mutex> lock(b->dev->mu);
+        auto& all = b->dev->batches;
+        all.erase(std::remove(all.begin(), all.end(), b), all.end());
+    }
     if (b->stream) cudaStreamSynchronize(b->stream);
     cudaFree(b->d_x);
     cudaFree(b->d_t);
@@ -973,6 +1027,7 @@ void mm_b200_destroy(mm_b200_batch* b) {
     if (b->d_items) cudaFree(b->d_items);
     if (b->h_items) cudaFreeHost(b->h_items);
     if (b->items_copied) cudaEventDestroy(b->items_copied);
+    if (b->paced) cudaEventDestroy(b->paced);
     delete b;
 }
 
@@ -1375,6 +1430,7 @@ int mm_b200_plan_run_async(mm_b200_plan* p, size_t bits) {
     MM_CK(cudaEventRecord(p->done, p->stream));
     for (auto* b : p->batches) {
         MM_CK(cudaStreamWaitEvent(b->stream, p->done, 0));
+        b->stepping = true;
         b->host_x_valid = false;
     }
     return MM_OK;
@@ -1427,6 +1483,7 @@ int mm_b200_plan_run_each_async(mm_b200_plan* p, const size_t* steps) {
     MM_CK(cudaEventRecord(p->done, p->stream));
     for (auto* b : p->batches) {
         MM_CK(cudaStreamWaitEvent(b->stream, p->done, 0));
+        b->stepping = true;
         b->host_x_valid = false;
     }
     return MM_OK;
@@ -1511,6 +1568,7 @@ int mm_b200_plan_run_items(mm_b200_plan* p, size_t count, const uint32_t* batch,
     MM_CK(cudaEventRecord(p->done, p->stream));
     for (auto* b : p->batches) {
         MM_CK(cudaStreamWaitEvent(b->stream, p->done, 0));
+        b->stepping = true;
         b->host_x_valid = false;
     }
     return mm_b200_plan_sync(p);

@@ -202,3 +202,64 @@ def test_bare_steps_in_rotation_leave_x_alone(gpu):
     be, st = b.backend_and_state()
     be.run_bare(st, steps)
     assert ran(b)["slots"] < slots and np.array_equal(raw(b), before) and b.remaining(0) == 0
+
+
+def test_wide_blocks_only_while_they_fit_beside_other_batches():
+    """L = 512: 64 slots run in 128-thread blocks alone and beside 64 more of the length, in the default
+    32-thread ones beside a batch of another length: with run while that one has steps under way, with run_async
+    (which cannot see what is enqueued after it) while it exists. The limbs are the same."""
+    from montmul_b200 import B200
+    dev = B200()
+    a, twin = batch(dev, 8_000, 64, [400] * 64), batch(dev, 8_000, 64, [400] * 64)
+    be, st = a.backend_and_state()
+    tst = twin.backend_and_state()[1]
+    be.set_schedule(tst, 0, 0, 0.0, 32)
+    twin.run(400)
+    seen = []
+
+    def step(run):
+        run(st, 50)
+        be.sync(st)
+        seen.append(ran(a)["threads"])
+
+    step(be.run)
+    step(be.run_async)
+    other = batch(dev, 100_000, 8, [4000] * 8)
+    ost = other.backend_and_state()[1]
+    step(be.run)
+    step(be.run_async)
+    be.run_async(ost, 4000)   # about 0.4 s
+    step(be.run)
+    assert be.busy(ost)
+    be.sync(ost)
+    step(be.run)
+    del other, ost
+    step(be.run_async)
+    step(be.run)
+    assert seen == [128, 128, 128, 32, 32, 128, 128, 128]
+    assert np.array_equal(raw(a), raw(twin))
+
+
+def test_batches_run_by_threads_keep_their_limbs():
+    """Four threads, each with its own batches, which come and go while the others run."""
+    import threading
+    from montmul_b200 import B200
+    dev = B200()
+    want = [batch(dev, bits, 40, [300] * 40) for bits in (4_000, 8_000, 16_000, 33_000)]
+    for b in want:
+        b.run(300)
+    got = [[] for _ in want]
+
+    def work(i, bits):
+        for _ in range(3):
+            b = batch(dev, bits, 40, [300] * 40)
+            b.run(300)
+            got[i].append(raw(b))
+
+    threads = [threading.Thread(target=work, args=(i, bits)) for i, bits in enumerate((4_000, 8_000, 16_000, 33_000))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for b, rows in zip(want, got):
+        assert len(rows) == 3 and all(np.array_equal(raw(b), r) for r in rows)
