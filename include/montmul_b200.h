@@ -188,7 +188,9 @@ void mm_b200_t_free(mm_b200_tbuf *b);
  * the launches of run when a batch has so few slots that SMs would idle; L = 4096,
  * 8192 and 16384 also build one alternative shape); in cluster mode, threads per SM (0 or 512:
  * one 512-thread block of 8192 elements per SM; 1024 at L = 32768: two 512-thread blocks of 4096
- * elements per SM, a cluster of 4). get_schedule reports the schedule: its mode and its block shape,
+ * elements per SM, a cluster of 4). A schedule's mode holds; without one (or force_global), run steps
+ * L = 131072 in clusters of eight blocks where that is faster. set_launch changes launch_steps and
+ * step_ns and names no mode or shape. get_schedule reports the schedule: its mode and its block shape,
  * which item lists and plans run; last_run reports what run's launches took. The autotuner
  * (montmul_b200.tune) measures these per length and caches them. */
 typedef struct {
@@ -198,6 +200,7 @@ typedef struct {
     int threads;
 } mm_b200_schedule;
 int mm_b200_set_schedule(mm_b200_batch *b, const mm_b200_schedule *s);
+int mm_b200_set_launch(mm_b200_batch *b, int launch_steps, double step_ns);
 int mm_b200_get_schedule(const mm_b200_batch *b, mm_b200_schedule *s);
 /* What the launches of the batch's last run, run_async or run_bare with steps to do took: mode (as
  * in the schedule), threads per block, blocks per slot (cluster mode; else 1), and the most slots

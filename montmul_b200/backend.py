@@ -68,6 +68,7 @@ SIGNATURES = {
     "mm_b200_busy": ([_vp], C.c_int),
     "mm_b200_bfly_peak": ([C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)], C.c_int),
     "mm_b200_set_schedule": ([_vp, _vp], C.c_int),
+    "mm_b200_set_launch": ([_vp, C.c_int, C.c_double], C.c_int),
     "mm_b200_get_schedule": ([_vp, _vp], C.c_int),
     "mm_b200_last_run": ([_vp, _vp], C.c_int),
     "mm_b200_set_moduli": ([_vp, _sz, _vp, _vp, _vp], C.c_int),
@@ -238,7 +239,7 @@ class B200:
                 self._table = tune.load_table()
             sc = tune.schedule_for(self.device_name(), length, self._table, self.wraparound)
             if sc:
-                self.set_schedule(st, sc["global"], sc["launch_steps"], sc["step_ns"], sc.get("block_threads", 0))
+                self.apply_row(st, sc, sc["step_ns"])
         return st
 
     def load(self, st, i, limbs):
@@ -375,10 +376,22 @@ class B200:
         sc = Schedule(int(global_mode), int(launch_steps), float(step_ns), int(threads))
         _check(lib().mm_b200_set_schedule(st.ptr, C.byref(sc)))
 
+    def set_launch(self, st, launch_steps: int = 0, step_ns: float = 0.0):
+        """launch_steps and step_ns of the batch's schedule; names no mode or block shape."""
+        _check(lib().mm_b200_set_launch(st.ptr, int(launch_steps), float(step_ns)))
+
+    def apply_row(self, st, row, step_ns: float):
+        """A row of the schedule table. One that keeps the batch's mode and default block shape names
+        neither, so that run may still choose (wide blocks, clusters of eight at L = 131072)."""
+        if int(row["global"]) == self.get_schedule(st)["number"] and not row.get("block_threads", 0):
+            self.set_launch(st, row["launch_steps"], step_ns)
+        else:
+            self.set_schedule(st, row["global"], row["launch_steps"], step_ns, row.get("block_threads", 0))
+
     def get_schedule(self, st):
         sc = Schedule()
         _check(lib().mm_b200_get_schedule(st.ptr, C.byref(sc)))
-        return {"global": bool(sc.global_), "mode": ("shared", "global", "cluster")[sc.global_],
+        return {"global": bool(sc.global_), "number": sc.global_, "mode": ("shared", "global", "cluster")[sc.global_],
                 "launch_steps": sc.launch_steps, "step_ns": sc.step_ns, "threads": sc.threads}
 
     def last_run(self, st):

@@ -98,6 +98,7 @@ struct mm_b200_batch {
     bool step_fixed = false;   // the schedule names the block shape: no wide shape in its place
     bool global = false;       // vector in HBM, tiles through shared memory (mm_global.cuh)
     bool cluster = false;      // global batch stepped in cluster mode (mm_cluster.cuh)
+    bool mode_fixed = false;   // the caller named the mode (a schedule, or force_global)
     int cluster_chunk_log = kClusterChunkLog;   // elements per block of the cluster: 2^13 or 2^12
     const DevTables* ctab = nullptr;   // shared-layout tables of a cluster-mode length
     bool plain = false;        // REDC without the wraparound path (k may be below L/2)
@@ -313,8 +314,11 @@ int ensure_cluster(mm_b200_batch* b) {
 // device holds 18 such clusters, 432 us a step, so 24 us per slot-step at any number of slots;
 // global mode takes 4.1 ms a step for up to one slot per SM and 22 us per slot-step from two per
 // SM on. The clusters are faster up to one slot per SM (24 slots x 8 steps: 35.2 -> 6.9 ms) and
-// slower beyond. The plain REDC path has no cluster form; the mixed launch's items stay in global mode.
-bool cluster_capable(const mm_b200_batch* b) { return b->global && !b->cluster && b->m == kClusterWideLogN && !b->plain; }
+// slower beyond. The plain REDC path has no cluster form, the mixed launch's items stay in global mode,
+// and so does a batch whose caller named that mode.
+bool cluster_capable(const mm_b200_batch* b) {
+    return b->global && !b->cluster && !b->mode_fixed && b->m == kClusterWideLogN && !b->plain;
+}
 
 // Blocks of a shared-memory step kernel that the batch's device holds at once.
 int resident_blocks(mm_b200_batch* b, StepFn fn, int threads, int* out) {
@@ -741,6 +745,7 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     b->base = base;
     b->tab = tab;
     b->global = global;
+    b->mode_fixed = dev->force_global;
     b->plain = !dev->wrap;
     b->sched.global = global ? 1 : 0;
     b->gk = global_kernels();
@@ -1073,6 +1078,7 @@ int mm_b200_set_schedule(mm_b200_batch* b, const mm_b200_schedule* sc) {
     b->global = global;
     b->cluster = cluster;
     b->cluster_chunk_log = chunk_log;
+    b->mode_fixed = true;
     if (!global) {
         b->step_fn = fn;
         b->step_threads = threads;
@@ -1081,6 +1087,14 @@ int mm_b200_set_schedule(mm_b200_batch* b, const mm_b200_schedule* sc) {
     b->sched = *sc;
     b->sched.global = cluster ? 2 : (global ? 1 : 0);
     b->sched.threads = global ? (cluster ? (chunk_log == kClusterChunkLog ? 512 : 1024) : b->gk.threads) : threads;
+    return MM_OK;
+}
+
+int mm_b200_set_launch(mm_b200_batch* b, int launch_steps, double step_ns) {
+    if (!b) return fail(MM_ERR_ARG, "set_launch: null batch");
+    if (launch_steps < 0 || step_ns < 0) return fail(MM_ERR_ARG, "set_launch: negative value");
+    b->sched.launch_steps = launch_steps;
+    b->sched.step_ns = step_ns;
     return MM_OK;
 }
 

@@ -27,17 +27,12 @@ def main(argv=None):
     dev = B200(max_launch_steps=a.steps)
     b = ModBatch(dev, moduli, 3)
     be, st = b.backend_and_state()
-    shape = 0
     if a.mode == "tuned":
         row = tune.schedule_for(dev.device_name(), b.params.len)
-        mode = int(row["global"]) if row else None
-        shape = int(row.get("block_threads", 0)) if row else 0
+        if row:
+            be.apply_row(st, dict(row, launch_steps=a.steps), 0.0)
     else:
-        mode = {"shared": tune.SHARED, "global": tune.GLOBAL, "cluster": tune.CLUSTER}[a.mode]
-    if mode is not None:
-        be.set_schedule(st, mode, a.steps, 0.0, shape)
-    sc = be.get_schedule(st)
-    print(f"L = {b.params.len}, mode {sc['mode']}, {sc['threads']} threads, {a.steps} steps per launch")
+        be.set_schedule(st, {"shared": tune.SHARED, "global": tune.GLOBAL, "cluster": tune.CLUSTER}[a.mode], a.steps)
     arm(b, exps)
     for i in range(a.launches):
         t = time.perf_counter()
@@ -45,6 +40,9 @@ def main(argv=None):
         dt = time.perf_counter() - t
         print(f"launch {i}: {a.slots} slots x {a.steps} steps in {dt * 1e3:.1f} ms "
               f"({a.slots * a.steps / dt:.0f} modsq/s)")
+    ran = be.last_run(st)
+    print(f"L = {b.params.len}, mode {ran['mode']}, {ran['threads']} threads, {ran['blocks']} blocks per slot, "
+          f"{ran['slots']} slots and up to {a.steps} steps per launch")
     return 0
 
 

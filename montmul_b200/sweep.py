@@ -73,12 +73,12 @@ def one_size(dev, bits: int, slots: int, ebits: int, seed: int = 2026) -> dict:
             if b.read(out) != x * y % moduli[out]:
                 raise MontMulError(f"{bits} bits: mul disagrees")
             muls += 1
-    sched = be.get_schedule(st)
+    ran = be.last_run(st)
     n = length // 2
     rate = slots * e_bits / secs
     return {"bits": bits, "L": length, "slots": slots, "ebits": e_bits, "seconds": secs, "modsq_per_s": rate,
             "bitsteps_per_s": rate * bits, "gbfly_per_s": rate * butterfly_pairs(n) / 1e9,
-            "mode": sched["mode"], "tuned": tuned, "mul_checked": muls, "timed_runs": len(runs),
+            "mode": ran["mode"], "tuned": tuned, "mul_checked": muls, "timed_runs": len(runs),
             "clocks": clk.summary()}
 
 

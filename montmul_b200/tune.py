@@ -242,7 +242,7 @@ def apply(batch, table=None) -> bool:
     sc = schedule_for(be.device_name(), batch.params.len, table, getattr(be, "wraparound", True))
     if not sc:
         return False
-    be.set_schedule(st, sc["global"], sc["launch_steps"], sc.get("mixed_ns", sc["step_ns"]), sc.get("block_threads", 0))
+    be.apply_row(st, sc, sc.get("mixed_ns", sc["step_ns"]))
     return True
 
 

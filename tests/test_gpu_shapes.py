@@ -204,6 +204,48 @@ def test_bare_steps_in_rotation_leave_x_alone(gpu):
     assert ran(b)["slots"] < slots and np.array_equal(raw(b), before) and b.remaining(0) == 0
 
 
+def test_a_named_mode_holds_at_131072(gpu, oracle):
+    """Clusters of eight are run's own choice: a schedule that names global mode, and force_global, keep it (and
+    the global kernel its oracle comparison at this length); a tuned row in the batch's mode names none."""
+    from montmul_b200 import B200
+    forced = B200(force_global=True)
+
+    class Named:
+        def __getattr__(self, name):
+            return getattr(gpu, name)
+
+        def create(self, *a):
+            st = gpu.create(*a)
+            gpu.set_schedule(st, 1)
+            return st
+
+    class Checked:
+        """Asserts after every run that it took global mode."""
+
+        def __init__(self, dev):
+            self.dev = dev
+
+        def __getattr__(self, name):
+            return getattr(self.dev, name)
+
+        def run(self, st, bits):
+            self.dev.run(st, bits)
+            assert self.dev.last_run(st)["mode"] == "global"
+
+    for dev in (Checked(forced), Checked(Named())):
+        common.same_raw(lambda: dev, oracle.OracleBackend.wraparound, 16 * 131072 - 4, 2, 3)
+    b = batch(gpu, 2_000_000, 1, [4])
+    b.run(1)
+    assert ran(b)["mode"] == "cluster"
+    tune.apply(b, {gpu.device_name(): {"131072": {"global": 1, "launch_steps": 64, "step_ns": 2e4}}})
+    b.run(1)
+    assert ran(b)["mode"] == "cluster"
+    be, st = b.backend_and_state()
+    be.set_schedule(st, 1)
+    b.run(1)
+    assert ran(b)["mode"] == "global"
+
+
 def test_wide_blocks_only_while_they_fit_beside_other_batches():
     """L = 512: 64 slots run in 128-thread blocks alone and beside 64 more of the length, in the default
     32-thread ones beside a batch of another length: with run while that one has steps under way, with run_async
