@@ -99,6 +99,7 @@ struct mm_b200_batch {
     bool global = false;       // vector in HBM, tiles through shared memory (mm_global.cuh)
     bool cluster = false;      // global batch stepped in cluster mode (mm_cluster.cuh)
     bool mode_fixed = false;   // the caller named the mode (a schedule, or force_global)
+    int clusters = 0;          // clusters of eight the device holds, where run may choose them (L = 131072)
     int cluster_chunk_log = kClusterChunkLog;   // elements per block of the cluster: 2^13 or 2^12
     const DevTables* ctab = nullptr;   // shared-layout tables of a cluster-mode length
     bool plain = false;        // REDC without the wraparound path (k may be below L/2)
@@ -154,10 +155,19 @@ int ensure_tables(mm_b200_device* dev, int m, bool global, const DevTables** out
         std::vector<F2K> t2 = host::karatsuba_form(global ? host::gen_global_length_tables<F2>(m) : host::gen_length_tables<F2>(m));
         std::vector<F1> t1 = global ? host::gen_global_length_tables<F1>(m) : host::gen_length_tables<F1>(m);
         DevTables d;
-        MM_CK(cudaMalloc(&d.t2, t2.size() * sizeof(F2K)));
-        MM_CK(cudaMalloc(&d.t1, t1.size() * sizeof(F1)));
-        MM_CK(cudaMemcpy(d.t2, t2.data(), t2.size() * sizeof(F2K), cudaMemcpyHostToDevice));
-        MM_CK(cudaMemcpy(d.t1, t1.data(), t1.size() * sizeof(F1), cudaMemcpyHostToDevice));
+        const auto upload = [&]() -> int {
+            MM_CK(cudaMalloc(&d.t2, t2.size() * sizeof(F2K)));
+            MM_CK(cudaMalloc(&d.t1, t1.size() * sizeof(F1)));
+            MM_CK(cudaMemcpy(d.t2, t2.data(), t2.size() * sizeof(F2K), cudaMemcpyHostToDevice));
+            MM_CK(cudaMemcpy(d.t1, t1.data(), t1.size() * sizeof(F1), cudaMemcpyHostToDevice));
+            return MM_OK;
+        };
+        const int rc = upload();
+        if (rc) {   // create may go on without a second table set
+            cudaFree(d.t2);
+            cudaFree(d.t1);
+            return rc;
+        }
         d.inv8h2 = host::inv8h<F2>(m);
         d.inv8h1 = host::inv8h<F1>(m);
         it = dev->tables.emplace(key, d).first;
@@ -314,7 +324,7 @@ int ensure_cluster(mm_b200_batch* b) {
 // device holds 18 such clusters, 432 us a step, so 24 us per slot-step at any number of slots;
 // global mode takes 4.1 ms a step for up to one slot per SM and 22 us per slot-step from two per
 // SM on. The clusters are faster up to one slot per SM (24 slots x 8 steps: 35.2 -> 6.9 ms) and
-// slower beyond. The plain REDC path has no cluster form, the mixed launch's items stay in global mode,
+// slower beyond (clusters_pay). The plain REDC path has no cluster form, the mixed launch's items stay in global mode,
 // and so does a batch whose caller named that mode.
 bool cluster_capable(const mm_b200_batch* b) {
     return b->global && !b->cluster && !b->mode_fixed && b->m == kClusterWideLogN && !b->plain;
@@ -378,17 +388,26 @@ int wide_shape(mm_b200_batch* b, size_t active, const WideShape** out) {
     return MM_OK;
 }
 
+// Clusters of the batch's length that the device holds at once.
+int resident_clusters(mm_b200_batch* b, int* out) {
+    std::lock_guard<std::mutex> lock(b->dev->mu);
+    auto it = b->dev->resident_clusters.find(32 * b->m + b->cluster_chunk_log);
+    if (it == b->dev->resident_clusters.end()) {
+        int held = 0;
+        const int e = cluster_capacity(b->m, b->cluster_chunk_log, &held);
+        if (e) return fail(MM_ERR_CUDA, std::string("cluster mode: ") + cudaGetErrorString((cudaError_t)e));
+        it = b->dev->resident_clusters.emplace(32 * b->m + b->cluster_chunk_log, held).first;
+    }
+    *out = it->second;
+    return MM_OK;
+}
+
 // Slots (blocks, clusters) that one launch of run keeps on the device at once.
 int resident_slots(mm_b200_batch* b, bool clustered, StepFn fn, int threads, size_t* out) {
     int n = 0;
     if (clustered) {
-        std::lock_guard<std::mutex> lock(b->dev->mu);
-        int& held = b->dev->resident_clusters[32 * b->m + b->cluster_chunk_log];
-        if (!held) {
-            const int e = cluster_capacity(b->m, b->cluster_chunk_log, &held);
-            if (e) return fail(MM_ERR_CUDA, std::string("cluster mode: ") + cudaGetErrorString((cudaError_t)e));
-        }
-        n = held;
+        const int rc = resident_clusters(b, &n);
+        if (rc) return rc;
     } else if (b->global) {
         n = 2 * b->dev->sms;   // gstep_kernel: 96 KiB of shared memory and at most 128 registers a thread
     } else {
@@ -424,11 +443,7 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
         g = global_args(b);
         g.a.bare = a.bare;
     }
-    const bool clustered = b->cluster || (cluster_capable(b) && active <= (size_t)b->dev->sms);
-    if (clustered) {
-        rc = ensure_cluster(b);
-        if (rc) return rc;
-    }
+    const bool clustered = b->cluster || (cluster_capable(b) && clusters_pay(active, b->dev->sms, b->clusters));
     SlotArgs c = a;   // cluster mode reads the shared-layout tables
     if (clustered) {
         c.tab2 = b->ctab->t2;
@@ -751,9 +766,9 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     b->gk = global_kernels();
     b->sched.threads = global ? b->gk.threads : (m <= kMaxSharedLogN ? threads_for(m) : 0);
     b->gtab = gtab;
-    if (cluster_capable(b.get())) {
-        rc = ensure_cluster(b.get());
-        if (rc) return rc;
+    if (cluster_capable(b.get()) && (ensure_cluster(b.get()) || resident_clusters(b.get(), &b->clusters))) {
+        cudaGetLastError();   // no second table set or no cluster launch: the length runs in global mode
+        b->clusters = 0;
     }
     if (m <= kMaxSharedLogN) {
         kernel_set(m, b->ks);

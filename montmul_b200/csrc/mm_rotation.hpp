@@ -14,6 +14,10 @@
 
 namespace mm {
 
+// Whether `active` slots of a length that global mode also runs are stepped in clusters, of which the
+// device holds `clusters` at once (none where its SMs are shared out in smaller groups).
+inline bool clusters_pay(size_t active, size_t sms, int clusters) { return clusters > 0 && active <= sms; }
+
 // The steps per launch with which `slots` slots of which `resident` fit the device at once finish
 // `steps` steps soonest when launches take the slots in rotation, `resident` at a time; 0 where one
 // launch over all slots is as good. That launch takes ceil(slots / resident) whole waves, the last

@@ -28,6 +28,10 @@ int main() {
             std::printf("%zu\n", mm::rotation_chunk(slots, resident, steps, last, step_us, launch_us, half_wave));
             continue;
         }
+        if (!std::strcmp(what, "clusters")) {   // "clusters active sms clusters 0"
+            std::printf("%d\n", (int)mm::clusters_pay(slots, resident, (int)steps));
+            continue;
+        }
         if (!std::strcmp(what, "pays")) {
             size_t chunk;
             double step_us, launch_us;
@@ -181,3 +185,7 @@ def test_half_full_last_wave_at_8192(ask):
     for slots, rotates in ((301, True), (370, True), (444, False), (540, True), (800, True), (1006, False)):
         assert (chunk(slots, 0.53) > 0) == rotates, slots
     assert all(chunk(slots, 1) > 0 for slots in (301, 370, 444, 540, 800, 1006))
+
+
+def test_clusters_need_room_for_one(ask):
+    assert ask("clusters 24 148 18 0 clusters 148 148 18 0 clusters 149 148 18 0 clusters 24 148 0 0") == ["1", "1", "0", "0"]
