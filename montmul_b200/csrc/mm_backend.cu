@@ -319,6 +319,9 @@ int ensure_cluster(mm_b200_batch* b) {
     return MM_OK;
 }
 
+// Bytes of the second table set (the shared-memory layout) that clusters of eight read.
+size_t cluster_table_bytes(int m) { return m == kClusterWideLogN ? (size_t)lt_size(m) * (sizeof(F2K) + sizeof(F1)) : 0; }
+
 // L = 131072 in global mode can also step in clusters of eight blocks (mm_cluster.cuh), the vector in
 // their shared memory, where global mode takes one block per slot and streams it through HBM. A
 // device holds 18 such clusters, 432 us a step, so 24 us per slot-step at any number of slots;
@@ -711,12 +714,12 @@ size_t mm_b200_batch_bytes(size_t slots, size_t len, size_t exp_words) {
     const size_t n = len / 2;
     // x (4n), T (8n), constants F(N') and A|B (2n elements of 24 B), exponent words, nbits,
     // pos and err, per slot; plus mul's spectrum scratch (24n) and this length's tables. Global
-    // mode (n > 8192) adds the per-slot work vector (24n).
+    // mode (n > 8192) adds the per-slot work vector (24n), L = 131072 the tables of its clusters.
     const int m = log2_exact(n);
     const bool global = m > kMaxSharedLogN;
     const size_t per_slot = 4 * n + 8 * n + 48 * n + (global ? 24 * n : 0) + 4 * exp_words + 12;
     const size_t tabs = m < kMinLogN ? 0 : (size_t)(global ? glt_size(m) : lt_size(m)) * (sizeof(F2K) + sizeof(F1));
-    return slots * per_slot + 24 * n + tabs;
+    return slots * per_slot + 24 * n + tabs + cluster_table_bytes(m);
 }
 
 int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, size_t slots, const uint32_t* n,
@@ -735,7 +738,8 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     // batch_bytes counts global mode's work vectors from n > 8192 on; forced global mode below
     // that adds them here.
     const size_t forced = global && m <= kMaxSharedLogN ? 24 * slots * k : 0;
-    const size_t need = mm_b200_batch_bytes(slots, len, 1) + 8 * slots * k + forced + ((size_t)64 << 20);
+    // The second table set is left out where it does not fit.
+    const size_t need = mm_b200_batch_bytes(slots, len, 1) - cluster_table_bytes(m) + 8 * slots * k + forced + ((size_t)64 << 20);
     const size_t freeb = mm_b200_free_memory(dev);
     if (need > freeb) return fail(MM_ERR_OOM, "batch needs " + std::to_string(need) + " bytes, " + std::to_string(freeb) + " free");
     // Shared-mode tables for every length that has them (mul_noalloc and schedule switches read

@@ -47,6 +47,26 @@ def test_limits_without_device():
     assert per_slot == (4 + 8 + 48 + 24) * (1 << 15) + 4 + 12
 
 
+def test_batch_bytes_counts_the_cluster_tables(tmp_path):
+    """L = 131072 has a second table set, in the shared-memory layout (lt_size, mm_common.h): 32 + 8 bytes an entry."""
+    import shutil
+    import subprocess
+    from montmul_b200 import backend
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include "mm_common.h"\n#include <cstdio>\n#include <initializer_list>\nint main() { for (int m : {15, 16, 17}) '
+                   'std::printf("%d %d\\n", mm::glt_size(m), mm::lt_size(m)); }\n')
+    subprocess.run([gxx, "-std=c++17", "-I", os.path.join(ROOT, "montmul_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    rows = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()
+    for m, row in zip((15, 16, 17), rows):
+        glob, shared = map(int, row.split())
+        n = 1 << m
+        tables = backend.lib().mm_b200_batch_bytes(1, 2 * n, 1) - ((4 + 8 + 48 + 24) * n + 16) - 24 * n
+        assert tables == 40 * (glob + (shared if m == 16 else 0))
+
+
 # The reference's launch planner (montmul/src/gpu/plan.rs:26-64), restated to pin the mode
 # boundary: shared mode when the vector (24 B per complex element) and the carry scratch fit the
 # device's opt-in shared memory per block, else global mode.
