@@ -10,7 +10,9 @@
 // swz(j), a permutation within aligned 16-element blocks); upload and download apply and remove it
 // on the device. Coefficients cross the bus as the caller's 32-bit limbs and become field elements on
 // the device: 64 vectors of L = 8,192 through load_forward twice, pointwise, inverse and
-// download_raw, 19.0 ms with the host expanding and permuting them, take 5.7.
+// download_raw take 3.8 ms where the host expanding and permuting them took 13.9 (medians of 200 passes
+// of one process; on a shared host single passes and whole processes vary by more than that). The rest is
+// the 6.3 MB result into fresh pages and the allocations.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -70,18 +72,23 @@ __global__ void pointwise_kernel(F2* o2, F1* o1, const F2* a2, const F1* a1, con
 
 // Field elements of a buffer from rows of k 32-bit coefficients, zero from k on (cpu.rs:349-358):
 // coefficient j in the real part of element j, j + n in the imaginary part, as it is for M61 and mod
-// M31. SWZ: the buffer is in the kernels' element order.
+// M31. SWZ: the buffer is in the kernels' element order. The rows are in the memory that the M31 elements
+// will take (8 bytes an element, the 4 bytes of two coefficients), so the M31 elements are made from
+// the M61 ones by a second kernel.
 template <bool SWZ>
-__global__ void expand_kernel(const uint32_t* __restrict__ c, uint32_t k, int logn, size_t total, F2* o2, F1* o1) {
+__global__ void expand_kernel(const uint32_t* __restrict__ c, uint32_t k, int logn, size_t total, F2* o2) {
     const uint32_t n = 1u << logn;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const size_t v = e >> logn;
         const uint32_t j = (uint32_t)e & (n - 1);
         const uint32_t* row = c + v * k;
-        const uint32_t re = j < k ? row[j] : 0u, im = j + n < k ? row[j + n] : 0u;
-        const size_t at = SWZ ? (v << logn) + (size_t)swz((int)j) : e;
-        o2[at] = f2(re, im);
-        o1[at] = f1(csubp1((re & P1) + (re >> 31)), csubp1((im & P1) + (im >> 31)));
+        o2[SWZ ? (v << logn) + (size_t)swz((int)j) : e] = f2(j < k ? row[j] : 0u, j + n < k ? row[j + n] : 0u);
+    }
+}
+__global__ void expand_m31_kernel(const F2* __restrict__ in, size_t total, F1* o1) {
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t re = (uint32_t)in[e].re, im = (uint32_t)in[e].im;
+        o1[e] = f1(csubp1((re & P1) + (re >> 31)), csubp1((im & P1) + (im >> 31)));
     }
 }
 
@@ -102,8 +109,8 @@ struct DevMem {
     ~DevMem() { cudaFree(p); }
 };
 
-// Bounds of the device staging of an upload (32-bit words) and of a global-mode download (elements).
-constexpr size_t kStageWords = (size_t)16 << 20, kStageElements = (size_t)1 << 20;
+// Bound of the device staging of a global-mode download, in elements.
+constexpr size_t kStageElements = (size_t)1 << 20;
 
 bool swizzled(size_t n) { return log2_len(n) > kMaxSharedLogN; }
 
@@ -122,21 +129,16 @@ int upload_rows(mm_b200_device* dev, const uint32_t* rows, size_t k, size_t len,
     b->n = n;
     TK(cudaMalloc(&b->d2, std::max<size_t>(1, total) * sizeof(F2)));
     TK(cudaMalloc(&b->d1, std::max<size_t>(1, total) * sizeof(F1)));
-    // Vectors per staged copy of rows.
-    const size_t step = k ? std::max<size_t>(1, std::min(count, kStageWords / k)) : count;
-    DevMem raw;
-    if (total) TK(cudaMalloc(&raw.p, std::max<size_t>(1, step * k) * 4));
-    for (size_t v0 = 0; v0 < count; v0 += step) {
-        const size_t vs = std::min(step, count - v0), part = vs * n;
-        if (k) TK(cudaMemcpyAsync(raw.p, rows + v0 * k, vs * k * 4, cudaMemcpyHostToDevice, cudaStreamLegacy));
-        const uint32_t* c = static_cast<const uint32_t*>(raw.p);
-        F2* o2 = b->d2 + v0 * n;
-        F1* o1 = b->d1 + v0 * n;
-        if (swizzled(n)) expand_kernel<true><<<grid_for(part), 256, 0, cudaStreamLegacy>>>(c, (uint32_t)k, l - 1, part, o2, o1);
-        else expand_kernel<false><<<grid_for(part), 256, 0, cudaStreamLegacy>>>(c, (uint32_t)k, l - 1, part, o2, o1);
+    if (total) {
+        uint32_t* c = reinterpret_cast<uint32_t*>(b->d1);
+        if (k) TK(cudaMemcpyAsync(c, rows, count * k * 4, cudaMemcpyHostToDevice, cudaStreamLegacy));
+        if (swizzled(n)) expand_kernel<true><<<grid_for(total), 256, 0, cudaStreamLegacy>>>(c, (uint32_t)k, l - 1, total, b->d2);
+        else expand_kernel<false><<<grid_for(total), 256, 0, cudaStreamLegacy>>>(c, (uint32_t)k, l - 1, total, b->d2);
         TK(cudaGetLastError());
+        expand_m31_kernel<<<grid_for(total), 256, 0, cudaStreamLegacy>>>(b->d2, total, b->d1);
+        TK(cudaGetLastError());
+        TK(cudaStreamSynchronize(cudaStreamLegacy));   // the caller's rows are free again
     }
-    if (total) TK(cudaStreamSynchronize(cudaStreamLegacy));   // the caller's rows and the staging are free again
     *out = b.release();
     return MM_OK;
 }
@@ -150,7 +152,20 @@ int download(const T* d, size_t n, size_t total, void* host) {
     }
     const size_t step = std::min(total, kStageElements);
     DevMem stage;
-    TK(cudaMalloc(&stage.p, step * sizeof(T)));
+    if (cudaMalloc(&stage.p, step * sizeof(T)) != cudaSuccess) {
+        // No room for the staging: the order is undone in place on the host (swz permutes within 16 elements).
+        cudaGetLastError();
+        stage.p = nullptr;
+        TK(cudaMemcpy(host, d, total * sizeof(T), cudaMemcpyDeviceToHost));
+        T* h = static_cast<T*>(host);
+        for (size_t e = 0; e < total; e += 16) {
+            T in[16];
+            std::copy(h + e, h + e + 16, in);
+            const int j0 = (int)(e & (n - 1));
+            for (int j = 0; j < 16; ++j) h[e + j] = in[swz_c(j0 + j) & 15];
+        }
+        return MM_OK;
+    }
     for (size_t e = 0; e < total; e += step) {
         const size_t part = std::min(step, total - e);
         natural_kernel<<<grid_for(part), 256, 0, cudaStreamLegacy>>>(d, log2_len(n), e, part, static_cast<T*>(stage.p));

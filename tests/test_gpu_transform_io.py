@@ -41,3 +41,28 @@ def test_load_forward_pads_with_zeros(gpu, length, k):
     gpu.forward(b, length, count)
     for x, y in zip(gpu.download_raw(a), gpu.download_raw(b)):
         assert np.array_equal(x, y)
+
+
+def test_upload_and_download_at_the_memory_limit(gpu):
+    """With room for the buffer and little else: the upload has no staging of its own, and a download whose staging
+    does not fit puts the elements in order on the host."""
+    import torch
+    length, count = 1 << 15, 512   # 192 MiB of elements from 64 MiB of coefficients
+    c = _coeffs(7, length * count)
+    small = gpu.upload(c[:length], length, 1)   # the kernels are loaded
+    gpu.download_raw(small)
+    torch.zeros(1, device="cuda")
+    torch.cuda.empty_cache()
+    fill = []
+    try:
+        fill.append(torch.empty(gpu.free_memory() - (226 << 20), dtype=torch.uint8, device="cuda"))
+        buf = gpu.upload(c, length, count)
+        room = gpu.free_memory() - (8 << 20)
+        if room > 0:
+            fill.append(torch.empty(room, dtype=torch.uint8, device="cuda"))
+        f1, f2 = gpu.download_raw(buf)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    want = c.reshape(count, 2, length // 2).transpose(0, 2, 1).reshape(-1, 2)
+    assert np.array_equal(f2, want.astype(np.uint64)) and np.array_equal(f1, want % P1)
