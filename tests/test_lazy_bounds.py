@@ -1,10 +1,6 @@
-"""The lazy GF(M61) arithmetic of the kernels never overflows 64 bits and keeps every value
-stored between passes below 2^61 + 2^34 (interval model in lazy_bounds_model.py). CPU only."""
+"""The lazy GF(M61) products of the kernels never overflow 64 bits and keep every value
+stored between passes below 2^61 + 2^34 (lazy_bounds_model.py; the butterflies: test_wrapped_bounds.py). CPU only."""
 import lazy_bounds_model as m
-
-
-def test_butterfly_bounds():
-    m.check_butterflies()
 
 
 def test_pointwise_bounds():
