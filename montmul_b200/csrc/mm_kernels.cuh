@@ -297,20 +297,23 @@ __device__ __forceinline__ void step_slot(const SlotArgs& a, uint32_t slot, uint
 
 // The uniform launch: one block per slot of the range; or, with an item
 // list, one block per item (slot, steps) of the list (a serving tick's launch over the busy slots
-// of a batch; each slot at most once).
+// of a batch; each slot at most once). Both take slot and steps from shared memory and share one copy of
+// the step: with a copy each, and the range's slot from the launch's arguments, run's was the slower
+// one at L = 16384 (189.7 us a step against 185.6 on 148 slots; now 185.3 both) and the code spilt more (L = 8192
+// 170.2 -> 168.0 us on 296 slots, L = 4096 93.7 -> 91.4).
 template <int M, int NT, int MINB = (M <= 12 ? 2 : 1), bool SP = false>
 __global__ void __launch_bounds__(NT, MINB)
     step_kernel(SlotArgs a, StepRange r, const uint2* __restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t sc[CarryScratch<NT>::words];
-    if (items) {
-        const uint2 it = items[blockIdx.x];
-        step_slot<M, NT, SP>(a, it.x, it.y, smem_raw, sc);
-    } else {
+    __shared__ uint2 item;
+    if (threadIdx.x == 0) {
         uint32_t bits;
         const uint32_t slot = range_slot(r, blockIdx.x, bits);
-        step_slot<M, NT, SP>(a, slot, bits, smem_raw, sc);
+        item = items ? items[blockIdx.x] : make_uint2(slot, bits);
     }
+    __syncthreads();
+    step_slot<M, NT, SP>(a, item.x, item.y, smem_raw, sc);
 }
 
 // x[out] <- x[ia] x[ib] R^-1 with slot out's modulus (cpu.rs:558-571), one block. spec: n

@@ -53,6 +53,8 @@ def radix_schedule(m: int):
     """Radix of every pass of a length-2^m transform (the device schedule, mm_common.h)."""
     if m <= 3:
         return [{1: 2, 2: 4, 3: 8}[m]] if m >= 1 else []
+    if m == 16:   # clusters of eight: after a radix-8 first pass every group lies inside one block
+        return [8, 4, 4, 8, 8, 8]
     if m % 3 == 0:
         return [8] * (m // 3)
     if m % 3 == 1:
@@ -171,6 +173,18 @@ def measure_mixed(dev, length: int, slots: int, steps: int, seed: int = 2026):
     return dt / (slots * steps)
 
 
+def pick(results):
+    """The fastest candidate; one that names a block shape only where it is 1 % faster than the default
+    shape, since a named shape keeps run from widening the blocks of batches with few slots."""
+    best = min(results, key=lambda r: r["step_ns"])
+    plain = [r for r in results if not r.get("block_threads")]
+    if best.get("block_threads") and plain:
+        default = min(plain, key=lambda r: r["step_ns"])
+        if default["step_ns"] < 1.01 * best["step_ns"]:
+            return default
+    return best
+
+
 def tune_length(dev, length: int, budget_s: float = 4.0):
     """The fastest schedule of one length, with every candidate's time."""
     sms = dev.sm_count()
@@ -184,8 +198,8 @@ def tune_length(dev, length: int, budget_s: float = 4.0):
     for g, s, th in cands:
         sec = measure(dev, length, g, s, slots, steps, threads=th)
         results.append({"global": g, "launch_steps": s, "block_threads": th, "step_ns": sec * 1e9})
-    ranked = sorted(results, key=lambda r: r["step_ns"])
-    best = ranked[0]
+    best = pick(results)
+    ranked = [best] + sorted((r for r in results if r is not best), key=lambda r: r["step_ns"])
     out = dict(best)
     if len(ranked) > 1:
         out["runner_up"] = dict(ranked[1])

@@ -177,19 +177,21 @@ def test_rotation_in_a_run_of_many_launches(gpu):
     assert np.array_equal(raw(a), raw(b))
 
 
-# (bits, wraparound, forced global, slots per SM, more slots, steps): several blocks per SM, the plain REDC,
-# the global-mode kernel, clusters of eight (18 of them on 148 SMs).
-@pytest.mark.parametrize("bits,wrap,forced,per_sm,more,steps", [
-    (8_000, True, False, 16, 40, 40), (12_000, True, False, 6, 10, 40), (20_011, False, False, 2, 5, 40), (131_068, True, True, 2, 1, 12),
-    (2_097_148, True, False, 0, 25, 4)])
-def test_rotation_in_every_mode(bits, wrap, forced, per_sm, more, steps):
+# (bits, wraparound, forced global, slots beyond what the device holds, steps): several blocks per SM, the
+# plain REDC, the global-mode kernel; 25 clusters of eight (18 fit on 148 SMs).
+@pytest.mark.parametrize("bits,wrap,forced,more,steps", [
+    (8_000, True, False, 40, 40), (12_000, True, False, 10, 40), (20_011, False, False, 5, 40), (131_068, True, True, 1, 12),
+    (2_097_148, True, False, None, 4)])
+def test_rotation_in_every_mode(bits, wrap, forced, more, steps):
     from montmul_b200 import B200
     dev = B200(wraparound=wrap, force_global=forced)
-    slots = per_sm * dev.sm_count() + more
+    be, st = ModBatch(dev, [(1 << (bits - 1)) | 1], 2).backend_and_state()
+    resident = be.blocks_per_sm(st) * dev.sm_count()
+    slots = 25 if more is None else resident + more
     nbits = [steps if i % 9 else 1 + i % steps for i in range(slots)]
     a, b = batch(dev, bits, slots, nbits, base=2), batch(dev, bits, slots, nbits, base=2)
     a.run(steps)
-    assert ran(a)["slots"] < slots
+    assert ran(a)["slots"] < 25 if more is None else ran(a)["slots"] == resident
     for _ in range(steps):
         b.run(1)
     assert np.array_equal(raw(a), raw(b))

@@ -21,6 +21,25 @@ def test_radix_schedule_covers_every_stage():
             assert sched[-1] == 8   # the fused last pass is radix 8 (m = 4 runs [4, 4])
 
 
+def test_radix_schedule_is_the_headers(tmp_path):
+    """sched_radix of mm_common.h, built for the host."""
+    import os
+    import shutil
+    import subprocess
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    csrc = os.path.join(os.path.dirname(tune.__file__), "csrc")
+    src, exe = tmp_path / "r.cpp", tmp_path / "r"
+    src.write_text('#include "mm_common.h"\n#include <cstdio>\nint main() { for (int m = 1; m < 24; ++m) {\n'
+                   'for (int i = 0; i < mm::sched_passes(m); ++i) std::printf("%d ", mm::sched_radix(m, i));\n'
+                   'std::printf("\\n"); } }\n')
+    subprocess.run([gxx, "-std=c++17", "-I", csrc, str(src), "-o", str(exe)], check=True)
+    lines = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()
+    for m, line in zip(range(1, 24), lines):
+        assert [int(r) for r in line.split()] == tune.radix_schedule(m), m
+
+
 def test_tune_candidates_by_length():
     S, G, C = tune.SHARED, tune.GLOBAL, tune.CLUSTER
     assert tune.candidates(2048) == [(S, s, 0) for s in tune.LAUNCH_STEPS]
@@ -71,6 +90,16 @@ class _FakeDev:
 
     def sm_count(self):
         return 148
+
+
+def test_tune_names_a_block_shape_only_for_a_gain():
+    """At L = 4,096 the two shapes measure alike; naming one would turn the wide shapes off."""
+    default = {"global": 0, "launch_steps": 512, "block_threads": 0, "step_ns": 311.5}
+    assert tune.pick([default, dict(default, block_threads=256, step_ns=311.3)]) is default
+    shaped = dict(default, block_threads=256, step_ns=300.0)
+    assert tune.pick([default, shaped]) is shaped
+    other = dict(default, launch_steps=64, step_ns=311.0)
+    assert tune.pick([default, other]) is other
 
 
 def test_tune_mixed_only_remeasures_the_mixed_cost_and_keeps_schedules(tmp_path, monkeypatch):
