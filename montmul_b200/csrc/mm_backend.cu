@@ -333,14 +333,14 @@ bool cluster_capable(const mm_b200_batch* b) {
     return b->global && !b->cluster && !b->mode_fixed && b->m == kClusterWideLogN && !b->plain;
 }
 
-// Blocks of a shared-memory step kernel that the batch's device holds at once.
-int resident_blocks(mm_b200_batch* b, StepFn fn, int threads, int* out) {
+// Blocks of a step kernel that the batch's device holds at once.
+int resident_blocks(mm_b200_batch* b, const void* fn, int threads, int smem, int* out) {
     std::lock_guard<std::mutex> lock(b->dev->mu);
-    auto it = b->dev->resident.find((const void*)fn);
+    auto it = b->dev->resident.find(fn);
     if (it == b->dev->resident.end()) {
         int per = 0;
-        MM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, b->ks.smem));
-        it = b->dev->resident.emplace((const void*)fn, per * b->dev->sms).first;
+        MM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem));
+        it = b->dev->resident.emplace(fn, per * b->dev->sms).first;
     }
     *out = it->second;
     return MM_OK;
@@ -381,7 +381,7 @@ int wide_shape(mm_b200_batch* b, size_t active, const WideShape** out) {
     for (const WideShape& w : b->ks.wide) {
         if (!w.step) continue;
         int res = 0;
-        const int rc = resident_blocks(b, w.step, w.threads, &res);
+        const int rc = resident_blocks(b, (const void*)w.step, w.threads, b->ks.smem, &res);
         if (rc) return rc;
         if (active <= (size_t)std::min(res, 5 * b->dev->sms)) {
             *out = &w;
@@ -411,10 +411,9 @@ int resident_slots(mm_b200_batch* b, bool clustered, StepFn fn, int threads, siz
     if (clustered) {
         const int rc = resident_clusters(b, &n);
         if (rc) return rc;
-    } else if (b->global) {
-        n = 2 * b->dev->sms;   // gstep_kernel: 96 KiB of shared memory and at most 128 registers a thread
     } else {
-        const int rc = resident_blocks(b, fn, threads, &n);
+        const int rc = b->global ? resident_blocks(b, (const void*)b->gk.step, b->gk.threads, b->gk.smem, &n)
+                                 : resident_blocks(b, (const void*)fn, threads, b->ks.smem, &n);
         if (rc) return rc;
     }
     *out = (size_t)std::max(1, n);
@@ -482,7 +481,7 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
     // A step of one launch's resident slots: the schedule's time per slot-step at full occupancy
     // times their number, else a model of the transform work.
     const double step_us = b->sched.step_ns > 0 ? 1e-3 * b->sched.step_ns * (double)resident : 1e-3 * (double)b->n * b->m;
-    const double launch_us = b->global ? 13.0 : 90.0;
+    const double launch_us = b->global ? 13.0 : b->m == kMaxSharedLogN ? 40.0 : 30.0;
     const double half_wave = !b->global && step_fn == b->ks.step && b->m == 12 ? 0.53 : 1.0;
     size_t turn = rotation_chunk(active, resident, left, chunk, step_us, launch_us, half_wave);
     if (turn && 8 * work < 7 * b->slots * left) {   // exponents of different lengths

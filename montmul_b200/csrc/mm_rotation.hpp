@@ -24,8 +24,10 @@ inline bool clusters_pay(size_t active, size_t sms, int clusters) { return clust
 // one of which may leave most SMs idle (37 clusters of L = 65536 where 36 fit: two waves for the
 // work of one); in rotation the idle places go to the next round's slots and only the last launch
 // is partly empty. A launch costs launch_us beyond its steps (its start, and the wait for its slowest
-// block), so a chunk is no shorter than pays for that: 13 us measured for clusters (one block per
-// SM), about 90 us in shared memory, where an SM's blocks finish at different times. The chunks
+// block), so a chunk is no shorter than pays for that: 13 us measured for clusters, 0 to 26 us in shared
+// memory (L = 1,024, 905 slots on 888 places: 5 launches of 2 steps 631 us, 9 of 8 4,133, a step is 57; L =
+// 8,192, 301 on 296: 17 of 4 11,550, 33 of 2 11,790, a step is 166), 30 to 48 us with one block per SM (L =
+// 16,384: 395 slots x 64 in 11 launches 33.4 ms, in 43 34.3; 503 x 256 in 17 165.3, in 109 170.6). The chunks
 // tried are those of 64 numbers of rounds, from the fewest that `most` steps per launch allow: past
 // that the last launch's idle places no longer count.
 // half_wave: a step of a launch that fills at most half the places, of a full one's. 1 where a step is as
@@ -112,6 +114,11 @@ class Rotation {
     bool next(const uint32_t* pos, const uint32_t* nbits, StepRange* r, size_t* count) {
         while (round_ * chunk_ < steps_) {
             size_t n = 0, live = 0, at = slot_, round = round_;
+            if (resident_ >= slots_) {   // a whole round: any slot with steps left will do
+                for (; n < slots_ && !live; ++n) live += pos[n] < nbits[n];
+                n = slots_;
+                ++round;
+            }
             while (n < slots_ && live < resident_ && round * chunk_ < steps_) {
                 live += pos[at] < nbits[at];
                 ++n;
@@ -131,11 +138,12 @@ class Rotation {
 
     // What the launch does to pos.
     static void advance(const StepRange& r, size_t count, uint32_t* pos, const uint32_t* nbits) {
-        for (size_t i = 0; i < count; ++i) {
-            uint32_t bits;
-            const uint32_t s = range_slot(r, (uint32_t)i, bits);
-            pos[s] += std::min(bits, nbits[s] - pos[s]);
-        }
+        const auto step = [&](size_t from, size_t to, uint32_t bits) {
+            for (size_t s = from; s < to; ++s) pos[s] += std::min(bits, nbits[s] - pos[s]);
+        };
+        const size_t end = r.first + count;
+        step(r.first, std::min<size_t>(end, r.slots), r.bits);
+        if (end > r.slots) step(0, end - r.slots, r.bits_next);
     }
 
   private:
