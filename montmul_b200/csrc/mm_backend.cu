@@ -752,10 +752,6 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     // On a failure below, everything allocated so far is released with the batch.
     std::unique_ptr<mm_b200_batch, void (*)(mm_b200_batch*)> b(new mm_b200_batch(), mm_b200_destroy);
     b->dev = dev;
-    {
-        std::lock_guard<std::mutex> lock(dev->mu);
-        dev->batches.push_back(b.get());
-    }
     b->m = m;
     b->k = k;
     b->n = len / 2;
@@ -832,6 +828,10 @@ int mm_b200_create(mm_b200_device* dev, size_t k, size_t len, uint32_t base, siz
     b->exps.assign(slots, std::vector<uint32_t>());
     b->nbits.assign(slots, 0);
     b->pos.assign(slots, 0);
+    {
+        std::lock_guard<std::mutex> lock(dev->mu);
+        dev->batches.push_back(b.get());   // complete: other threads' runs may look at it (slots_beside)
+    }
     *out = b.release();
     return MM_OK;
 }
@@ -1093,7 +1093,10 @@ int mm_b200_set_schedule(mm_b200_batch* b, const mm_b200_schedule* sc) {
         int rc = ensure_cluster(b);
         if (rc) return rc;
     }
-    b->global = global;
+    {
+        std::lock_guard<std::mutex> lock(b->dev->mu);   // slots_beside of other batches reads it
+        b->global = global;
+    }
     b->cluster = cluster;
     b->cluster_chunk_log = chunk_log;
     b->mode_fixed = true;
