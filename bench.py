@@ -41,15 +41,25 @@ def g_of_n(n: int) -> int:
 # dram__bytes_read.sum + dram__bytes_write.sum of one step_kernel launch of this workload, from
 # one ncu capture of `python -m montmul_b200.profile --slots SLOTS --steps STEPS --launches 2`
 # (second launch): the slots and steps per launch it ran, and its DRAM bytes.
-TRAFFIC_CAPTURE = {"slots": 2368, "steps_per_launch": 64, "dram_bytes": 13403741696 + 8097713920}
+TRAFFIC_CAPTURE = {"slots": 2368, "steps_per_launch": 64, "dram_bytes": 7375781376 + 3662561024}
 
 # The step kernel against the hardware, from one ncu capture of step_kernel<12, 512> on this
 # workload (296 slots x 16 steps, second launch): issue slots used, ALU pipe (integer add, logic,
 # shift, min: 2 cycles per warp instruction on a B200) and FMA-heavy pipe (IMAD, IMAD.WIDE)
-# cycles active. The integer pipes of a B200 SM (measured with single-instruction chains: 64
-# ALU-pipe and 64 IMAD lanes per clock) are the ceiling the butterfly peak below runs against.
-HW_CAPTURE = {"issue_active": 0.540, "alu_pipe": 0.556, "fmaheavy_pipe": 0.555, "warps_per_scheduler": 6.78,
+# cycles active.
+HW_CAPTURE = {"issue_active": 0.592, "alu_pipe": 0.597, "fmaheavy_pipe": 0.631, "warps_per_scheduler": 6.70,
               "capture": "ncu of step_kernel<12, 512>, 296 slots x 16 steps"}
+
+# The rate that butterfly pairs are reported against: one radix-2 pair's arithmetic (bfly_peak_kernel: 61
+# ALU-pipe and 41 IMAD-pipe instructions, 16 of them wide) takes 118 cycles of a warp's scheduler when spread
+# evenly over both integer pipes (2 cycles an instruction, 4 a wide product). A reference rate, not a bound: the
+# kernels' radix-8 passes need fewer instructions per pair, their carries and CRT others on top.
+PAIR_CYCLES = 118
+
+
+def pair_rate(sms: int, sm_mhz: float) -> float:
+    """Pairs per second of four schedulers per SM at PAIR_CYCLES per warp."""
+    return sms * 4 * 32 * sm_mhz * 1e6 / PAIR_CYCLES
 
 # The uneven-size persistent batch: 2,000 slots, bits log-uniform in [8,192, 300,000] (seed 7),
 # c in {2, 3, 4}, the top 1,000 bits of N - 1; the plan replays its launch from a CUDA graph
@@ -374,7 +384,8 @@ def main(argv=None):
     # Rooflines of the step kernel (it is every launch in the timed region).
     n = 4096
     per_step_s = total / args.steps
-    peak_pairs, _ = bk.bfly_peak(local)
+    chain_pairs, _ = bk.bfly_peak(local)
+    peak_pairs = pair_rate(be.sm_count(), (clocks or {}).get("sm_mhz") or 1965.0)
     achieved_pairs = slots * EBITS * g_of_n(n) / per_step_s
     peaks = measured_peaks()
     hbm = peaks.get("hbm_gbs")
@@ -388,18 +399,19 @@ def main(argv=None):
     same = cap["slots"] == slots and abs(cap["steps_per_launch"] - steps_per_launch) < 0.5
     traffic = cap["dram_bytes"] * (1.0 if same else slots * steps_per_launch / (cap["slots"] * cap["steps_per_launch"]))
     roofline = {"bound": "int", "achieved": achieved_pairs / 1e9, "peak": peak_pairs / 1e9, "unit": "Gbfly/s",
-                "frac": achieved_pairs / peak_pairs, "traffic": traffic,
+                "frac": achieved_pairs / peak_pairs, "chain": chain_pairs / 1e9, "traffic": traffic,
                 "traffic_note": ("dram__bytes_read+write per launch, measured by ncu on a launch of this size"
                                  if same else
                                  "dram__bytes_read+write of an ncu capture of %d slots x %d steps per launch, "
                                  "scaled to this run's %d slots x %.0f steps per launch (estimate)"
                                  % (cap["slots"], cap["steps_per_launch"], slots, steps_per_launch)),
                 "note": "butterfly pairs (GF(p^2) product + add + sub in both fields), G(n)=%d per modsq at "
-                        "L=8192; peak = the kernels' own arithmetic in register-resident chains on all SMs, "
-                        "measured in this run" % g_of_n(n)}
+                        "L=8192; peak = one pair's instructions spread over both integer pipes at %d cycles per "
+                        "warp and the sampled SM clock, a reference rate (radix-8 passes need fewer per pair, "
+                        "carries and CRT are not counted); chain = the pair as register-resident chains, measured "
+                        "in this run" % (g_of_n(n), PAIR_CYCLES)}
     roofline_hw = dict(HW_CAPTURE, note="fractions of the SM's issue slots and integer pipes the step kernel used "
-                                         "in an ncu capture; the butterfly roofline above counts the same arithmetic "
-                                         "against a register-resident chain of it")
+                                         "in an ncu capture: the distance to the hardware")
     roofline_hbm = {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm, "unit": "GB/s",
                     "frac": (achieved_gbs / hbm) if hbm else None,
                     "note": "48n B of per-slot constants per slot-step; peak of measured (MEASURED_PEAKS.json)"}

@@ -118,7 +118,7 @@ uint64_t mm_b200_launches(const mm_b200_batch *b);
  * to steps[i] steps (each slot at most once, steps[i] >= 1), and returns; mm_b200_sync waits and
  * reports errors as run does. Lists of several batches on their own streams run on the device
  * at the same time. Shared-memory lengths only (L <= 16384). blocks_per_sm: blocks of the
- * batch's step kernel that one SM holds at once (0 on an error). */
+ * schedule's step kernel (which item lists run) that one SM holds at once (0 on an error). */
 int mm_b200_run_items_async(mm_b200_batch *b, size_t count, const size_t *slots, const uint32_t *steps);
 int mm_b200_blocks_per_sm(const mm_b200_batch *b);
 /* 1 while work enqueued on the batch's stream is still running, 0 once it has finished (then
@@ -185,8 +185,9 @@ void mm_b200_t_free(mm_b200_tbuf *b);
  * launch of run (0: the device default). step_ns: the measured time of one slot-step at full
  * occupancy, which orders the items of a mixed launch (0: a model of the transform work).
  * threads: threads per block of the shared-memory step kernel (0: the length's default, or more in
- * the launches of run when a batch has so few slots that SMs would idle; L = 4096,
- * 8192 and 16384 also build one alternative shape); in cluster mode, threads per SM (0 or 512:
+ * the launches of run and run_bare while a batch and those stepping beside it have so few slots that
+ * SMs would idle, of run_async while all batches of the device have; L = 4096, 8192 and 16384 also
+ * build one alternative shape); in cluster mode, threads per SM (0 or 512:
  * one 512-thread block of 8192 elements per SM; 1024 at L = 32768: two 512-thread blocks of 4096
  * elements per SM, a cluster of 4). A schedule's mode holds; without one (or force_global), run steps
  * L = 131072 in clusters of eight blocks where that is faster. set_launch changes launch_steps and
@@ -265,8 +266,8 @@ uint64_t mm_b200_plan_launches(const mm_b200_plan *p);
 uint64_t mm_b200_plan_graph_launches(const mm_b200_plan *p);
 void mm_b200_plan_destroy(mm_b200_plan *p);
 
-/* Integer roofline probe (no counterpart in the reference, whose roofline is not measured):
- * the peak rate of butterfly pairs (a GF(p^2) product, an add and a sub in both fields) of the
+/* Integer probe (no counterpart in the reference, whose roofline is not measured): the
+ * rate of butterfly pairs (a GF(p^2) product, an add and a sub in both fields) of the
  * kernels' arithmetic from register-resident chains on every SM of `device`; `iters` chain
  * steps per thread. Writes pairs per second and the timed kernel's milliseconds. */
 int mm_b200_bfly_peak(int device, int iters, double *pairs_per_s, double *ms);

@@ -383,7 +383,8 @@ class B200:
     def apply_row(self, st, row, step_ns: float):
         """A row of the schedule table. One that keeps the batch's mode and default block shape names
         neither, so that run may still choose (wide blocks, clusters of eight at L = 131072)."""
-        if int(row["global"]) == self.get_schedule(st)["number"] and not row.get("block_threads", 0):
+        mode = ("shared", "global", "cluster")[int(row["global"])]
+        if mode == self.get_schedule(st)["mode"] and not row.get("block_threads", 0):
             self.set_launch(st, row["launch_steps"], step_ns)
         else:
             self.set_schedule(st, row["global"], row["launch_steps"], step_ns, row.get("block_threads", 0))
@@ -391,7 +392,7 @@ class B200:
     def get_schedule(self, st):
         sc = Schedule()
         _check(lib().mm_b200_get_schedule(st.ptr, C.byref(sc)))
-        return {"global": bool(sc.global_), "number": sc.global_, "mode": ("shared", "global", "cluster")[sc.global_],
+        return {"global": bool(sc.global_), "mode": ("shared", "global", "cluster")[sc.global_],
                 "launch_steps": sc.launch_steps, "step_ns": sc.step_ns, "threads": sc.threads}
 
     def last_run(self, st):

@@ -326,8 +326,9 @@ size_t cluster_table_bytes(int m) { return m == kClusterWideLogN ? (size_t)lt_si
 // their shared memory, where global mode takes one block per slot and streams it through HBM. A
 // device holds 18 such clusters, 432 us a step, so 24 us per slot-step at any number of slots;
 // global mode takes 4.1 ms a step for up to one slot per SM and 22 us per slot-step from two per
-// SM on. The clusters are faster up to one slot per SM (24 slots x 8 steps: 35.2 -> 6.9 ms) and
-// slower beyond (clusters_pay). The plain REDC path has no cluster form, the mixed launch's items stay in global mode,
+// SM on. The clusters are faster up to one slot per SM (24 slots x 8 steps: 35.2 -> 6.9 ms), which is where
+// the line lies (clusters_pay), still faster at 200 slots (two batches of 100 at once, 6 steps: 30 against 37 ms)
+// and slower at two per SM (42.9 against 40.2). The plain REDC path has no cluster form, the mixed launch's items stay in global mode,
 // and so does a batch whose caller named that mode.
 bool cluster_capable(const mm_b200_batch* b) {
     return b->global && !b->cluster && !b->mode_fixed && b->m == kClusterWideLogN && !b->plain;
@@ -366,15 +367,19 @@ size_t slots_beside(mm_b200_batch* b, bool alive) {
 }
 
 // The wide block shape for `active` slots in shared memory: the widest one whose blocks are all
-// resident at once, at most five per SM; none where the schedule fixes the shape. With
-// every slot resident the time of a run is one slot's, which more threads shorten (ms for 500 steps
-// at L = 512, default 32 threads -> wide: 64 slots 22.5 -> 14.5, 592 slots 23.4 -> 16.8; 300 steps at L = 1024,
-// 592 slots: 18.2 -> 13.7; 200 steps at L = 4096, 148 slots: 13.8 -> 10.7). With more slots the default
-// shape's rate per SM is higher (L = 512, 64 threads: 700 slots 24 -> 18.1, 1,000 slots 24.2 -> 26.8).
-// Slots of other batches that run at the same time count like the batch's own (slots_beside; four batches of 148
-// slots at L = 1024, 300 steps each under run_async: 24.8 ms in the default shape, 36.6 in wide ones).
-// Item lists (run_items) always take the default shape: a serving loop runs several of them at the
-// same time.
+// resident at once, at most five per SM; none where the schedule fixes the shape. With every slot resident
+// the time of a run is one slot's, which more threads shorten. us a step, default -> wide, for 1, 148, 592 and 740 slots:
+//   L = 128   32.4 -> 26.3  32.1 -> 29.6  32.1 -> 30.0  32.1 -> 30.5
+//   L = 256   34.4 -> 27.6  33.7 -> 30.1  34.6 -> 30.4  34.7 -> 31.2
+//   L = 512   47.2 -> 29.6  46.8 -> 32.8  47.8 -> 33.4  47.9 -> 36.7
+//   L = 1024  51.7 -> 39.1  51.2 -> 43.0  55.7 -> 45.8  (740: default)
+//   L = 2048  54.6 -> 36.2  54.1 -> 37.6  (296: 60.3 -> 59.8; from 297: default)
+//   L = 4096  70.2 -> 52.1  69.8 -> 53.2  (from 149: default)
+// With more slots the default shape's rate per SM is higher (L = 512, 64 threads: 700 slots 24 -> 18.1 ms for
+// 500 steps, 1,000 slots 24.2 -> 26.8). Slots of other batches that run at the same time count like the
+// batch's own (slots_beside; four batches of 148 slots at L = 1024, 300 steps each under run_async: 24.8 ms
+// in the default shape, 36.6 in wide ones). Item lists (run_items) always take the default shape: a serving
+// loop runs several of them at the same time.
 int wide_shape(mm_b200_batch* b, size_t active, const WideShape** out) {
     *out = nullptr;
     if (b->step_fixed || b->global) return MM_OK;
@@ -420,7 +425,9 @@ int resident_slots(mm_b200_batch* b, bool clustered, StepFn fn, int threads, siz
     return MM_OK;
 }
 
-// Steps per launch of a run in a wide shape that waits for its launches.
+// Steps per launch of a run in a wide shape that waits for its launches: 3 to 7 ms each. Two threads that run
+// 148 slots at L = 4096 each, 600 steps: 57.4 ms with 64 steps, 58.6 with 128, 65.4 with 256, 78.6 with 512 (default
+// shape 61.3); a batch alone is 0.1 to 0.3 % slower with 128 than with everything enqueued at once.
 constexpr size_t kPacedSteps = 128;
 
 // Enqueues up to `bits` steps on every slot. `waits`: the caller waits for them. A run that may take a wide
