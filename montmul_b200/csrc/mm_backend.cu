@@ -441,8 +441,6 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
     }
     const size_t left = std::min(bits, most);
     if (left == 0) return MM_OK;
-    size_t work = 0;
-    for (size_t i = 0; i < b->slots; ++i) work += std::min(left, (size_t)(b->nbits[i] - b->pos[i]));
     int rc = push(b);
     if (rc) return rc;
     SlotArgs a = slot_args(b);
@@ -459,7 +457,8 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
         c.tab1 = b->ctab->t1;
     }
     const WideShape* wide = nullptr;
-    rc = wide_shape(b, active + (waits ? 0 : slots_beside(b, true)), &wide);
+    rc = wide_shape(b, active, &wide);
+    if (!rc && wide && !waits) rc = wide_shape(b, active + slots_beside(b, true), &wide);
     if (rc) return rc;
     const bool paced = wide && waits;
     if (paced && !b->paced) MM_CK(cudaEventCreateWithFlags(&b->paced, cudaEventDisableTiming));
@@ -491,10 +490,15 @@ int launch_steps(mm_b200_batch* b, size_t bits, bool bare, bool waits) {
     const double launch_us = b->global ? 13.0 : b->m == kMaxSharedLogN ? 40.0 : 30.0;
     const double half_wave = !b->global && step_fn == b->ks.step && b->m == 12 ? 0.53 : 1.0;
     size_t turn = rotation_chunk(active, resident, left, chunk, step_us, launch_us, half_wave);
-    if (turn && 8 * work < 7 * b->slots * left) {   // exponents of different lengths
+    if (turn) {
         std::vector<uint32_t> rem(b->slots);
-        for (size_t i = 0; i < b->slots; ++i) rem[i] = (uint32_t)std::min(left, (size_t)(b->nbits[i] - b->pos[i]));
-        if (!rotation_pays(rem, resident, left, chunk, turn, step_us, launch_us)) turn = 0;
+        size_t work = 0;
+        for (size_t i = 0; i < b->slots; ++i) {
+            rem[i] = (uint32_t)std::min(left, (size_t)(b->nbits[i] - b->pos[i]));
+            work += rem[i];
+        }
+        // exponents of different lengths
+        if (8 * work < 7 * b->slots * left && !rotation_pays(rem, resident, left, chunk, turn, step_us, launch_us)) turn = 0;
     }
     // Without a rotation each launch takes every slot once.
     Rotation rot(b->slots, turn ? resident : b->slots, left, turn ? turn : std::min(left, chunk));
